@@ -121,6 +121,18 @@ struct DeviceMesh {
     uint32_t sched_cap = 0;
 };
 
+// Default launch configs: the ones the autotuner picked on GB300 for the displaced-icosphere frame
+// (single BLAS) and the instanced frame (two-level).
+inline bvhgpu_tune_config default_config(int kernel) {
+    const bool single = kernel == BVHGPU_K_TRACE_BLAS || kernel == BVHGPU_K_TRACE_SCENE;
+    return bvhgpu_tune_config{128u, 5u, 256u, 16u, single ? 1u : 8u, 2000u};
+}
+inline bool default_tune(const bvhgpu_tune_config& c, int kernel) {
+    const bvhgpu_tune_config d = default_config(kernel);
+    return c.block == d.block && c.min_blocks == d.min_blocks && c.stack == d.stack && c.big_leaf == d.big_leaf &&
+           c.refill == d.refill && c.hidden == d.hidden;
+}
+
 struct ProfileRec {
     int kernel;
     cudaEvent_t start, stop;
@@ -178,11 +190,7 @@ struct bvhgpu_ctx {
     // launch configuration per kernel id (only the tunable kernels read theirs)
     bvhgpu_tune_config tune[BVHGPU_KERNEL_COUNT];
     bvhgpu_ctx() {
-        // defaults: the configs the autotuner picked on GB300 for the displaced-icosphere frame
-        // (single BLAS) and the instanced frame (two-level)
-        for (auto& t : tune) t = bvhgpu_tune_config{128u, 5u, 256u, 16u, 8u, 2000u};
-        tune[BVHGPU_K_TRACE_BLAS].refill = 1u;
-        tune[BVHGPU_K_TRACE_SCENE].refill = 1u;
+        for (int k = 0; k < BVHGPU_KERNEL_COUNT; ++k) tune[k] = bvhgpu::default_config(k);
     }
 };
 

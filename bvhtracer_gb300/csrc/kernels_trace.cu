@@ -100,6 +100,206 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace_blas(GBlas b, const float
     if (active) store_hit(hits, out_index ? out_index[i] : i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, 0u);
 }
 
+// ---- one warp per ray ----------------------------------------------------------------------
+// For launches of few rays (wide_rays): one thread per ray leaves most of the GPU idle and its time
+// is one lane's walk, so here a warp takes one ray.  Every lane follows the same reference nodes in
+// the reference's order; a leaf is tested by all lanes at once, small leaves (or leaves whose margins
+// are too wide) in order as in coop_leaf, large ones through their hidden tree: up to 8 nodes' children
+// are tested per iteration, one box per lane, and the live leaves' pairs one per lane.  Any order
+// of testing inside a leaf is exact (smallest t, ties to the lowest index; a hit from an earlier leaf
+// keeps equal t out).  What bounds it: the latency of the dependent node loads of one ray.
+constexpr uint32_t kWideStack = 256;    // pending reference nodes, as the largest stack variant
+constexpr uint32_t kWideNodes = 224;    // pending hidden nodes; fuller: the leaf is tested in order
+constexpr uint32_t kWideLeaves = 96;    // live hidden leaves waiting to be tested
+constexpr int kWideWarps = 2;           // warps (rays) per block
+// Leaves of at most this many triangles are tested in order (8 rounds of 64).  4,000 camera rays
+// against a 4,096-triangle soup / a 20,480-triangle sphere: 13 / 15 us at 256, 512 and 1,024, 19 / 15
+// at 32, 13 / 27 at 1,500.
+constexpr uint32_t kWideInOrder = 512;
+
+struct WideSmem {
+    uint2 stack[kWideStack];
+    uint2 nodes[kWideNodes];
+    uint2 leaves[kWideLeaves];
+};
+
+// The warp's best hit of the leaf in every lane (smallest t, ties to the lowest index).
+__device__ __forceinline__ void wide_reduce(Best& b) {
+    // accepted t are positive, so their bits order as the values do; a lane without a hit holds the
+    // incoming t with index ~0
+    const uint32_t t = __reduce_min_sync(kFull, b.k == kMiss ? 0x7F800000u : __float_as_uint(b.t));
+    if (t == 0x7F800000u) return;
+    b.k = __reduce_min_sync(kFull, (b.k != kMiss && __float_as_uint(b.t) == t) ? b.k : kMiss);
+    b.t = __uint_as_float(t);
+}
+
+// Tests the leaf [first, first + cnt) in index order, pairs dealt over the lanes.
+__device__ __forceinline__ void wide_in_order(const GBlas& g, uint32_t first, uint32_t cnt, const LaneRay& r, Best& b) {
+    const unsigned lane = threadIdx.x & 31u;
+    const f2 OX = f2_pack(r.o.x, r.o.x), OY = f2_pack(r.o.y, r.o.y), OZ = f2_pack(r.o.z, r.o.z);
+    const f2 DX = f2_pack(r.d.x, r.d.x), DY = f2_pack(r.d.y, r.d.y), DZ = f2_pack(r.d.z, r.d.z);
+    const f2 Z = f2_neg_zero();
+    const uint32_t end = first + cnt;
+    for (uint32_t p = (first >> 1) + lane; p < (end + 1u) >> 1; p += 32u) {
+        const uint32_t kA = 2u * p;
+        const PairData pd = load_pair(g.pairs + 5ull * p);
+        b.take(ray_terms(pd, origin_terms(pd, OX, OY, OZ, Z), DX, DY, DZ, Z, kA >= first, kA + 1u < end), kA);
+    }
+}
+
+// Walks the hidden tree `root` under margins lc.  False: the node list overflowed (test in order).
+__device__ __forceinline__ bool wide_hidden(const GBlas& g, uint2 root, LeafCull& lc, const LaneRay& r, Best& b,
+                                            WideSmem& sm) {
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned below = (1u << lane) - 1u;
+    const uint2* hidx = g.hx + hidden_table_u2(g.ntris) - pairs_in_order(g.ntris);
+    const f2 OX = f2_pack(r.o.x, r.o.x), OY = f2_pack(r.o.y, r.o.y), OZ = f2_pack(r.o.z, r.o.z);
+    const f2 DX = f2_pack(r.d.x, r.d.x), DY = f2_pack(r.d.y, r.d.y), DZ = f2_pack(r.d.z, r.d.z);
+    const f2 Z = f2_neg_zero();
+    uint32_t nn = 1u, nl = 0u;
+    if (lane == 0u) sm.nodes[0] = make_uint2(root.y, root.x);  // (count, first)
+    __syncwarp();
+    while (nn | nl) {
+        if (nn && nl + 32u <= kWideLeaves) {
+            // the children of the newest up to 8 nodes, one box per lane
+            const uint32_t take = min(nn, 8u);
+            nn -= take;
+            const uint32_t slot = lane >> 2, c = lane & 3u;
+            bool live = false;
+            uint2 e = make_uint2(0u, 0u);
+            if (slot < take) {
+                const uint2 nd = sm.nodes[nn + slot];
+                if (c <= ((nd.x >> kWideShift) & 3u)) {
+                    const float4* N = g.nodes + 2ull * (nd.y + c);
+                    const float4 lo = __ldg(N), hi = __ldg(N + 1);
+                    float te;
+                    live = hidden_box(lo, hi, r.rd, lc, te);
+                    e = make_uint2(ubits(hi.w), ubits(lo.w));
+                }
+            }
+            const bool leaf = (e.x & kHiddenLeaf) != 0u;
+            const unsigned ml = __ballot_sync(kFull, live && leaf), mn = __ballot_sync(kFull, live && !leaf);
+            if (nn + (uint32_t)__popc(mn) > kWideNodes) return false;
+            __syncwarp();  // the entries taken above have been read
+            if (live && leaf) sm.leaves[nl + __popc(ml & below)] = e;
+            if (live && !leaf) sm.nodes[nn + __popc(mn & below)] = e;
+            nl += (uint32_t)__popc(ml);
+            nn += (uint32_t)__popc(mn);
+            __syncwarp();
+            if (nn && nl < 16u) continue;
+        }
+        // the newest up to 16 live leaves, one pair per lane (a hidden leaf has one or two)
+        const uint32_t take = min(nl, 16u);
+        if (take == 0u) continue;
+        nl -= take;
+        const uint32_t slot = lane >> 1;
+        if (slot < take) {
+            const uint2 e = sm.leaves[nl + slot];
+            if ((lane & 1u) < (e.x & ~kHiddenLeaf)) {
+                const uint32_t p = e.y + (lane & 1u);
+                const uint2 idx = __ldg(hidx + p);
+                const PairData pd = load_pair(g.pairs + 5ull * p);
+                const PairHit h = ray_terms(pd, origin_terms(pd, OX, OY, OZ, Z), DX, DY, DZ, Z, idx.x != kMiss, idx.y != kMiss);
+                if (h.okA && (h.tA < b.t || (h.tA == b.t && b.k != kMiss && idx.x < b.k))) {
+                    b.t = h.tA;
+                    b.k = idx.x;
+                }
+                if (h.okB && (h.tB < b.t || (h.tB == b.t && b.k != kMiss && idx.y < b.k))) {
+                    b.t = h.tB;
+                    b.k = idx.y;
+                }
+            }
+        }
+        __syncwarp();
+        wide_reduce(b);
+        lc.thi = leaf_thi(lc, b.t);
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(32 * kWideWarps) k_trace_wide(GBlas g, const float4* __restrict__ rays, uint32_t n,
+                                                                GHit* __restrict__ hits, LeafPolicy pol,
+                                                                uint32_t* err) {
+    __shared__ WideSmem smem[kWideWarps];
+    WideSmem& sm = smem[threadIdx.x >> 5];
+    const unsigned lane = threadIdx.x & 31u;
+    const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
+    if (i >= n) return;
+    LaneRay r;
+    float3 o, d;
+    float t0;
+    load_ray(rays, i, o, d, t0);
+    init_lane_ray(r, o, d, t0);
+    uint32_t cnt = g.root_count, first = g.root_first, sp = 0u, steps = 0u;
+    const uint32_t max_steps = 2u * (g.nodes_used + g.ntris) + 16u;
+    for (;;) {
+        if (++steps > max_steps) {
+            if (lane == 0u) atomicOr(err, kErrSteps);
+            break;
+        }
+        bool pop = true;
+        if (cnt == 0u) {
+            const float4* N = g.nodes + 2ull * first;
+            const float4 l0 = __ldg(N), l1 = __ldg(N + 1), r0 = __ldg(N + 2), r1 = __ldg(N + 3);
+            float dl, dr;
+            const bool hl = slab(l0, l1, r.o, r.rd, r.ct, dl), hr = slab(r0, r1, r.o, r.rd, r.ct, dr);
+            const bool left_near = (hl ? dl : FLT_MAX) < (hr ? dr : FLT_MAX);
+            if (left_near ? hl : hr) {
+                if (left_near ? hr : hl) {
+                    if (sp >= kWideStack) {
+                        if (lane == 0u) atomicOr(err, kErrStack);
+                        break;
+                    }
+                    if (lane == 0u)
+                        sm.stack[sp] = left_near ? make_uint2(ubits(r1.w), ubits(r0.w)) : make_uint2(ubits(l1.w), ubits(l0.w));
+                    ++sp;
+                    __syncwarp();
+                }
+                cnt = left_near ? ubits(l1.w) : ubits(r1.w);
+                first = left_near ? ubits(l0.w) : ubits(r0.w);
+                pop = false;
+            }
+        } else {
+            Best b{r.ct, kMiss};
+            bool done = false;
+            if (cnt > kWideInOrder && g.hx != nullptr && pol.max_duv > 0.0f) {
+                const uint2 e = __ldg(g.hx + first);
+                if (e.x != 0u) {
+                    const float4 a = __ldg(g.cones + 2ull * (e.y & kConeMask)), q = __ldg(g.cones + 2ull * (e.y & kConeMask) + 1);
+                    const LeafCone cone = {a.x, a.y, a.z, a.w, q.x, q.y};
+                    LeafCull lc = leaf_cull(cull_ray_rd(r.o.x, r.o.y, r.o.z, r.d.x, r.d.y, r.d.z, r.rd.x, r.rd.y, r.rd.z),
+                                            q.z, q.w, r.ct, pol.max_duv, cone);
+                    if (lc.on) {
+                        done = wide_hidden(g, e, lc, r, b, sm);
+                        if (!done) b = Best{r.ct, kMiss};
+                        __syncwarp();
+                    }
+                }
+            }
+            if (!done) wide_in_order(g, first, cnt, r, b);
+            wide_reduce(b);
+            if (b.k != kMiss) {
+                const float4* T = g.tris + 3ull * b.k;
+                float t, u, v;
+                tri_test(__ldg(T), __ldg(T + 1), __ldg(T + 2), r.o, r.d, t, u, v);  // the winner's u, v
+                r.ct = b.t;
+                r.hu = u;
+                r.hv = v;
+                r.hp = b.k;
+                r.hit = true;
+            }
+        }
+        if (pop) {
+            if (sp == 0u) break;
+            const uint2 e = sm.stack[--sp];
+            cnt = e.x;
+            first = e.y;
+            __syncwarp();
+        }
+    }
+    if (lane == 0u) store_hit(hits, i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, 0u);
+}
+
 // The plain traversal with per-ray work counters (one variant: block 128, local stack), summed
 // over the launch into out[0..6] in TraceCounts order -- the bytes each ray fetched, for the
 // roofline.  Results are the same as k_trace_blas's.
@@ -478,13 +678,33 @@ static cudaError_t trace_blas_variant(bvhgpu_ctx* ctx, const Variant& v, const G
     });
 }
 
+// Launches of at most this many rays run one warp per ray (under the default launch config only: a
+// config set by the caller or the tuner names the one-thread kernel's variants).  Measured against the
+// one-thread kernel, in us, at 8,000 / 16,000 / 32,000 / 64,000 camera rays (random rays gain more): soup of
+// 300 triangles 24 | 24 | 43 | 43 -> 23 | 37 | 85 | 143; sphere of 320 23 | 23 | 27 | 29 -> 16 | 25 |
+// 50 | 86; sphere of 5,120 58 | 72 | 72 | 74 -> 21 | 35 | 62 | 114; soup of 4,096 123 | 199 | 260 |
+// 293 -> 24 | 39 | 81 | 134; sphere of 81,920 194 | 203 | 203 | 248 -> 30 | 43 | 78 | 140.  The one-thread
+// kernel's time hardly grows until the GPU is full and then starts from the mesh's longest walk, so
+// the line lies higher for larger meshes.
+static uint32_t wide_rays(const bvhgpu_ctx* ctx, const DeviceBlas& b) {
+    if (!default_tune(ctx->tune[BVHGPU_K_TRACE_BLAS], BVHGPU_K_TRACE_BLAS)) return 0u;
+    return b.ntris < 4096u ? 8192u : 32768u;
+}
+
 cudaError_t launch_trace_blas(bvhgpu_ctx* ctx, const DeviceBlas& b, const float4* rays, uint32_t n, void* hits,
                               cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     GBlas g = to_gblas(b);
     LaunchScope scope(ctx, BVHGPU_K_TRACE_BLAS, s);
     const Variant v = resolve(ctx->tune[BVHGPU_K_TRACE_BLAS], b.depth);
-    cudaError_t e = trace_blas_variant(ctx, v, g, rays, n, nullptr, nullptr, static_cast<GHit*>(hits), s);
+    cudaError_t e;
+    if (n <= wide_rays(ctx, b)) {
+        k_trace_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(g, rays, n, static_cast<GHit*>(hits), v.pol,
+                                                                         ctx->d_err);
+        e = cudaGetLastError();
+    } else {
+        e = trace_blas_variant(ctx, v, g, rays, n, nullptr, nullptr, static_cast<GHit*>(hits), s);
+    }
     g_launches++;
     return e;
 }

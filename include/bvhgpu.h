@@ -469,7 +469,8 @@ typedef struct bvhgpu_tune_config {
     uint32_t hidden;
 } bvhgpu_tune_config;
 /* Defaults (the tuner's picks on GB300): block 128, min_blocks 5, stack 256, big_leaf 16, refill 8,
- * hidden 2000; for the single-ray kernels (TRACE_BLAS, TRACE_SCENE) refill 1. */
+ * hidden 2000; for the single-ray kernels (TRACE_BLAS, TRACE_SCENE) refill 1.  While TRACE_BLAS has its
+ * default config, launches of few rays run one warp per ray instead (same hits). */
 int bvhgpu_tune_get(bvhgpu_ctx* ctx, int kernel, bvhgpu_tune_config* out);
 /* BVHGPU_ERR_INVALID_ARG for a kernel that is not tunable or a shape / stack not compiled. */
 int bvhgpu_tune_set(bvhgpu_ctx* ctx, int kernel, const bvhgpu_tune_config* cfg);
