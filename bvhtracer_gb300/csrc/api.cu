@@ -1172,7 +1172,7 @@ int bvhgpu_scene_create(bvhgpu_ctx* ctx, const uint32_t* blas_ids, uint32_t nobj
         (e = cudaMalloc(&sc.obj_blas, 4ull * nobjects)) != cudaSuccess ||
         (e = cudaMalloc(&sc.blas_table, sizeof(GBlas) * table.size())) != cudaSuccess ||
         (e = cudaMalloc(&sc.tlas, 64ull * nobjects)) != cudaSuccess ||
-        (nobjects > kTlasSharedObjects && (e = cudaMalloc(&sc.tlas_work, tlas_smem_bytes(nobjects))) != cudaSuccess)) {
+        (nobjects > kTlasBlockObjects && (e = cudaMalloc(&sc.tlas_work, tlas_work_bytes(nobjects))) != cudaSuccess)) {
         free_scene(sc);
         return fail(ctx, BVHGPU_ERR_OUT_OF_MEMORY, "scene_create: %s", cudaGetErrorString(e));
     }

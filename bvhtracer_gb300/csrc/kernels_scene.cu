@@ -5,8 +5,8 @@
 // nodes bottom-up with one arrival counter per node: the second child to finish computes its
 // parent with the reference's min/max order (left child first).
 //
-// TLAS rebuild (Tlas::rebuild, tlas.rs:204-250): the reference's agglomerative clustering with
-// find_best_match results cached per list position in shared memory (see k_tlas_rebuild).
+// TLAS rebuild (Tlas::rebuild, tlas.rs:204-250): the reference's agglomerative clustering by one block
+// that keeps the list in registers (see k_tlas_rebuild).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -434,57 +434,36 @@ __global__ void __launch_bounds__(kBlock) k_refit_leaves(float4* nodes, const fl
 
 // ---- TLAS ------------------------------------------------------------------------------------
 // Tlas::rebuild (tlas.rs:204-250) walks nearest neighbours over a list of node indices and
-// calls find_best_match (tlas.rs:179-202) -- a full scan of the list -- at every step.  Here
-// each list position keeps the result find_best_match would give for it as one 64-bit key in
-// shared memory: the area's order-preserving rank (both zeros one rank) above the position, so
-// the smallest key is the smallest area with ties to the lower position, as the reference's
-// strict `<` scan from FLT_MAX keeps it; areas not below FLT_MAX (and NaN) are never keys.  A
-// merge updates only what it can change:
-//  - the merged node lands on position a, the last node moves to position b, the list shrinks;
-//  - a position whose cached best was a, b or the old last position is rescanned in full, by
-//    several warps at once (each a slice of the list, combined with a shared-memory atomicMin);
-//  - any other position keeps its cached best, which is still the first minimum over the
-//    positions whose node did not change, and compares it with the two changed positions.
-// The walk then reads the cache.  The TLAS is bit for bit Tlas::rebuild's, including the case
-// where position a itself leaves the list (its stale entry is then scanned like a rescan).
-
-constexpr int kTlasThreads = 512;
-// Above this many objects the rebuild scans instead of caching each position's best match: the
-// cache's rescans grow with the clusters (measured: 4,096 objects 2.5 s cached, 10 ms scanning;
-// 256 objects, the instanced frame's, 0.46 ms cached, 0.61 ms scanning).
-constexpr uint32_t kTlasCachedObjects = 256;
+// calls find_best_match (tlas.rs:179-202) -- a full scan of the list -- at every step, about three
+// times per merge.  The scans follow one another, so the rebuild's time is their number times the
+// latency of one.  Here one block keeps the list in registers (k_tlas_rebuild): thread t owns
+// clusters t, t + B, ..., a scan is one area per owned cluster, a warp minimum and a minimum over
+// the warps behind a single barrier, and a merge needs no barrier of its own.  A candidate is one
+// 64-bit key: the area's order-preserving rank (both zeros one rank) above the position, so the
+// smallest key is the smallest area with ties to the lower position, as the reference's strict `<`
+// scan from FLT_MAX keeps it; areas not below FLT_MAX (and NaN) are never keys.  The TLAS is bit for
+// bit Tlas::rebuild's, including the case where position a itself leaves the list.
 constexpr unsigned long long kNoKey = 0xFFFFFFFFFFFFFFFFull;
-
-struct TlasSmem {  // one entry per list position
-    unsigned long long* key;              // cached find_best_match(p)
-    float *lx, *ly, *lz, *hx, *hy, *hz;  // node bounds (nodes[list[p]].aabb)
-    int* node;                            // list[p]: node index
-    int* inval;                           // positions to rescan after a merge
-};
 
 struct Box6 {
     float lx, ly, lz, hx, hy, hz;
 };
-
-__device__ __forceinline__ Box6 load_box(const TlasSmem& S, int p) {
-    return Box6{S.lx[p], S.ly[p], S.lz[p], S.hx[p], S.hy[p], S.hz[p]};
-}
 
 // find_best_match's area (tlas.rs:184-193): component_max / component_min, then
 // ex*ey + ey*ez + ez*ex.  The area is only compared (as a key rank), never stored, so fmaxf /
 // fminf stand in for the first-operand-on-ties f32::max / f32::min: they ignore NaN the same way
 // and can differ only in the sign of a zero coordinate, which changes at most the sign of a zero
 // area -- the same rank.
-__device__ __forceinline__ float sa_merge(const Box6& a, const TlasSmem& S, int r) {
-    float ex = fsub(fmaxf(a.hx, S.hx[r]), fminf(a.lx, S.lx[r]));
-    float ey = fsub(fmaxf(a.hy, S.hy[r]), fminf(a.ly, S.ly[r]));
-    float ez = fsub(fmaxf(a.hz, S.hz[r]), fminf(a.lz, S.lz[r]));
+__device__ __forceinline__ float sa_merge(const Box6& a, const Box6& b) {
+    float ex = fsub(fmaxf(a.hx, b.hx), fminf(a.lx, b.lx));
+    float ey = fsub(fmaxf(a.hy, b.hy), fminf(a.ly, b.ly));
+    float ez = fsub(fmaxf(a.hz, b.hz), fminf(a.lz, b.lz));
     return fadd(fadd(fmul(ex, ey), fmul(ey, ez)), fmul(ez, ex));
 }
 
-// The cache key of candidate r for query box P (kNoKey where the reference would not take it).
-__device__ __forceinline__ unsigned long long sa_key(const Box6& P, const TlasSmem& S, int r) {
-    const float s = sa_merge(P, S, r);
+// The key of candidate r for query box P (kNoKey where the reference would not take it).
+__device__ __forceinline__ unsigned long long sa_key(const Box6& P, const Box6& R, int r) {
+    const float s = sa_merge(P, R);
     return s < FLT_MAX ? (((unsigned long long)ordered(s) << 32) | (uint32_t)r) : kNoKey;
 }
 
@@ -496,18 +475,6 @@ __device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k)
     const uint32_t hi = __reduce_min_sync(kFull, (uint32_t)(k >> 32));
     const uint32_t lo = __reduce_min_sync(kFull, (uint32_t)(k >> 32) == hi ? (uint32_t)k : 0xFFFFFFFFu);
     return ((unsigned long long)hi << 32) | lo;
-}
-
-// find_best_match for position p over positions [r0, r1) by one warp.
-__device__ __forceinline__ unsigned long long warp_best_key(const TlasSmem& S, int p, int r0, int r1) {
-    const Box6 P = load_box(S, p);
-    unsigned long long best = kNoKey;
-    for (int r = r0 + (int)(threadIdx.x & 31u); r < r1; r += 32) {
-        if (r == p) continue;
-        const unsigned long long k = sa_key(P, S, r);
-        best = k < best ? k : best;
-    }
-    return warp_min_key(best);
 }
 
 __device__ __forceinline__ void xf_point_g(const float* m, float x, float y, float z, float* out) {
@@ -522,11 +489,164 @@ __device__ __forceinline__ void store_tlas_node(float4* out, uint32_t i, const B
     out[2ull * i + 1] = make_float4(b.hx, b.hy, b.hz, __uint_as_float(blas));
 }
 
+// Object i's world bounds (SceneObject::set_transform, scene_object.rs:60-75).
+__device__ __forceinline__ Box6 object_bounds(const GBlas& b, const float* m) {
+    const float4 rlo = b.nodes[0], rhi = b.nodes[1];  // Bvh::bounds = nodes[0].aabb (bvh.rs:499-501)
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
+    float hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    for (int c = 0; c < 8; ++c) {
+        float p[3];
+        xf_point_g(m, (c & 1) ? rhi.x : rlo.x, (c & 2) ? rhi.y : rlo.y, (c & 4) ? rhi.z : rlo.z, p);
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = min_ni(lo[k], p[k]);
+            hi[k] = max_ni(hi[k], p[k]);
+        }
+    }
+    return Box6{lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
+}
+
+__device__ __forceinline__ Box6 merged_box(const Box6& a, const Box6& b) {  // Aabb::new of positions a and b
+    return Box6{min_ni(a.lx, b.lx), min_ni(a.ly, b.ly), min_ni(a.lz, b.lz),
+                max_ni(a.hx, b.hx), max_ni(a.hy, b.hy), max_ni(a.hz, b.hz)};
+}
+
+// An object or merged cluster in shared memory: its box and node index.
+struct Cluster {
+    Box6 box;
+    int node;
+};
+__device__ __forceinline__ Cluster load_cluster(const float4* sm, int slot) {
+    const float4 x = sm[2 * slot], y = sm[2 * slot + 1];
+    return Cluster{Box6{x.x, x.y, x.z, x.w, y.x, y.y}, __float_as_int(y.z)};
+}
+__device__ __forceinline__ void store_cluster(float4* sm, int slot, const Box6& b, int node) {
+    sm[2 * slot] = make_float4(b.lx, b.ly, b.lz, b.hx);
+    sm[2 * slot + 1] = make_float4(b.hy, b.hz, __int_as_float(node), 0.0f);
+}
+
+// The whole rebuild of up to B * K objects by one block.  A cluster keeps its slot for life (thread
+// slot % B owns it: box and list position in registers, a copy of the box in shared memory for the
+// queries); the reference's list moves are changes of positions only.  The walk is followed by every
+// thread (a, b and their clusters are block-uniform).  A shared cluster is read only between a scan's
+// barrier and the next one; a merge writes one, between the same barriers and without another
+// reader: the clusters at a and b are already in registers and the next query is the merged one.
+// status[0] gets nodes_used, status[1] an error (the reference would panic).
+template <int B, int K>
+__global__ void __launch_bounds__(B) k_tlas_rebuild(const GBlas* __restrict__ blas_table,
+                                                    const uint32_t* __restrict__ obj_blas,
+                                                    const float* __restrict__ xf, uint32_t nobj,
+                                                    float4* __restrict__ tlas_out, uint32_t* status) {
+    static_assert(B % 32 == 0 && B / 32 <= 32, "one lane per warp in the second reduction");
+    static_assert(B * K <= 65536, "16-bit positions and slots in a key");
+    constexpr uint32_t kNobody = 0xFFFFFFFFu, kRankMax = 0xFF7FFFFFu;  // kRankMax: FLT_MAX's rank
+    extern __shared__ float4 tsm[];
+    __shared__ unsigned long long s_best[2][B / 32];
+    const int n = (int)nobj, tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    Box6 own[K];
+    uint32_t ps[K];  // list position << 16 | slot
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        const int i = tid + j * B;
+        // no cluster (also after a merge): areas with this box are infinite or NaN
+        own[j] = Box6{0.0f, 0.0f, 0.0f, INFINITY, INFINITY, INFINITY};
+        ps[j] = 0xFFFF0000u | (uint32_t)i;
+        if (i < n) {
+            ps[j] = ((uint32_t)i << 16) | (uint32_t)i;
+            own[j] = object_bounds(blas_table[obj_blas[i]], xf + 16ull * i);
+            store_cluster(tsm, i, own[j], 1 + i);  // leaves at 1..nobj (tlas.rs:210-218)
+            store_tlas_node(tlas_out, 1u + (uint32_t)i, own[j], 0u, (uint32_t)i);
+        }
+    }
+    __syncthreads();
+    int count = n, used = 1 + n, buf = 0;
+    uint32_t err = 0;
+    uint64_t steps = 0;
+    const uint64_t max_steps = 4ull * nobj * nobj + 64;
+    // find_best_match with box P, leaving out the cluster whose (position, slot) is `self`: the
+    // candidate's (position, slot), kNobody if there is none
+    auto best = [&](const Box6& P, uint32_t self) {
+        unsigned long long k[K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            // the order-preserving rank of the area, both zeros one rank (-0 + 0 = +0); an area that is
+            // not below FLT_MAX ranks at or above kRankMax, NaN too (the canonical one, positive)
+            const int bits = __float_as_int(fadd(sa_merge(P, own[j]), 0.0f));
+            const uint32_t rank = (uint32_t)(bits ^ ((bits >> 31) | (int)0x80000000));
+            k[j] = ((unsigned long long)(ps[j] == self ? 0xFFFFFFFFu : rank) << 32) | ps[j];
+        }
+#pragma unroll
+        for (int s = 1; s < K; s *= 2)
+#pragma unroll
+            for (int j = 0; j + s < K; j += 2 * s) k[j] = k[j + s] < k[j] ? k[j + s] : k[j];
+        unsigned long long m = warp_min_key(k[0]);
+        if (lane == 0) s_best[buf][warp] = m;
+        __syncthreads();
+        m = warp_min_key(lane < B / 32 ? s_best[buf][lane] : kNoKey);
+        buf ^= 1;  // the other slots are free: every thread read them before this scan's barrier
+        return (uint32_t)(m >> 32) < kRankMax ? (uint32_t)m : kNobody;
+    };
+    // a and b are (position << 16 | slot); the position of a goes stale when a itself was the last
+    uint32_t a = 0u;
+    Cluster A = load_cluster(tsm, 0);
+    uint32_t b = best(A.box, a);
+    while (count > 1) {
+        if (b == kNobody || ++steps > max_steps) {
+            err = 1;
+            break;
+        }
+        const Cluster C = load_cluster(tsm, (int)(b & 0xFFFFu));
+        const uint32_t c = best(C.box, b);
+        if (a != c) {
+            a = b;
+            A = C;
+            b = c;
+            continue;
+        }
+        // node `used` = Aabb::new of a and b, LeftRightIndex::new(node a, node b) = a + (b << 16)
+        // (tlas.rs:18-22, 234-236); position a then holds it and position b the last one
+        // (tlas.rs:238-240), also when a itself is the last
+        const int last = count - 1, a_slot = (int)(a & 0xFFFFu), b_slot = (int)(b & 0xFFFFu);
+        const Box6 m = merged_box(A.box, C.box);
+        if (tid == 0) store_tlas_node(tlas_out, (uint32_t)used, m, (uint32_t)A.node + ((uint32_t)C.node << 16), 0u);
+        if (tid == a_slot % B) store_cluster(tsm, a_slot, m, used);
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            const int slot = tid + j * B;
+            if (slot == a_slot) own[j] = m;
+            if (slot == b_slot) own[j] = Box6{0.0f, 0.0f, 0.0f, INFINITY, INFINITY, INFINITY};
+            if ((ps[j] >> 16) == (uint32_t)last) ps[j] = (b & 0xFFFF0000u) | (uint32_t)slot;
+        }
+        A = Cluster{m, used};
+        count = last;
+        used += 1;
+        b = best(m, a);  // its barrier publishes the merged cluster
+    }
+    if (tid == 0) {
+        if (err == 0) {  // nodes[0] = nodes[list[a]] (tlas.rs:248); thread 0 wrote every inner node itself
+            const float4 r0 = tlas_out[2ull * A.node], r1 = tlas_out[2ull * A.node + 1];
+            tlas_out[0] = r0;
+            tlas_out[1] = r1;
+        }
+        status[0] = (uint32_t)used;
+        status[1] = err;
+    }
+}
+
+// Larger scenes: the same walk with the list in global memory (`work`), every scan by a block of 512.
+constexpr int kTlasThreads = 512;
+
+struct TlasList {  // one entry per list position
+    float *lx, *ly, *lz, *hx, *hy, *hz;  // node bounds (nodes[list[p]].aabb)
+    int* node;                            // list[p]: node index
+};
+
+__device__ __forceinline__ Box6 load_box(const TlasList& S, int p) {
+    return Box6{S.lx[p], S.ly[p], S.lz[p], S.hx[p], S.hy[p], S.hz[p]};
+}
+
 // One merge of the walk by warp 0's lanes 0-6 (each touches only its own array): lane c < 6 the
-// c-th coordinate array, lane 6 the node list.  Node `used` gets Aabb::new of positions a and b and
-// LeftRightIndex::new(node a, node b) = a + (b << 16) (tlas.rs:18-22, 234-236); position a then
-// holds it and position b the list's last node (tlas.rs:238-240).
-__device__ __forceinline__ void tlas_merge(const TlasSmem& S, int n, float4* tlas_out, int a, int b, int last, int used,
+// c-th coordinate array, lane 6 the node list.
+__device__ __forceinline__ void tlas_merge(const TlasList& S, int n, float4* tlas_out, int a, int b, int last, int used,
                                            int lane) {
     if (lane >= 7) return;
     // node `used` as 8 floats: lo.xyz, left_right, hi.xyz, blas (0 for an inner node)
@@ -546,178 +666,71 @@ __device__ __forceinline__ void tlas_merge(const TlasSmem& S, int n, float4* tla
     }
 }
 
-// One block.  Object world bounds (SceneObject::set_transform, scene_object.rs:60-75) in
-// parallel, the cache filled one warp per position, then the walk: every thread follows it
-// (it only reads the keys), warp 0 writes the merged nodes, all threads update the cache.
-// status[0] gets nodes_used, status[1] an error (the reference would panic).  The per-position
-// state lives in shared memory, or in `gwork` (global, same layout) for scenes too large for it.
-__global__ void __launch_bounds__(kTlasThreads) k_tlas_rebuild(const GBlas* __restrict__ blas_table,
-                                                               const uint32_t* __restrict__ obj_blas,
-                                                               const float* __restrict__ xf, uint32_t nobj,
-                                                               float4* __restrict__ tlas_out, uint32_t* status,
-                                                               unsigned long long* gwork) {
-    extern __shared__ unsigned long long tsm_keys[];
-    __shared__ int s_ninval;
-    __shared__ unsigned long long s_key_a;
+__global__ void __launch_bounds__(kTlasThreads) k_tlas_rebuild_large(const GBlas* __restrict__ blas_table,
+                                                                     const uint32_t* __restrict__ obj_blas,
+                                                                     const float* __restrict__ xf, uint32_t nobj,
+                                                                     float4* __restrict__ tlas_out, uint32_t* status,
+                                                                     float* work) {
+    __shared__ unsigned long long s_key;
     const int n = (int)nobj;
-    TlasSmem S;
-    S.key = gwork != nullptr ? gwork : tsm_keys;
-    float* f = reinterpret_cast<float*>(S.key + n);
-    S.lx = f;
-    S.ly = f + n;
-    S.lz = f + 2 * n;
-    S.hx = f + 3 * n;
-    S.hy = f + 4 * n;
-    S.hz = f + 5 * n;
-    S.node = reinterpret_cast<int*>(f + 6 * n);
-    S.inval = reinterpret_cast<int*>(f + 7 * n);
+    const TlasList S = {work,         work + n,     work + 2 * n, work + 3 * n,
+                        work + 4 * n, work + 5 * n, reinterpret_cast<int*>(work + 6 * n)};
     const int tid = (int)threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31, nwarps = (int)(blockDim.x >> 5);
-
     for (int i = tid; i < n; i += (int)blockDim.x) {
-        const GBlas& b = blas_table[obj_blas[i]];
-        float4 rlo = b.nodes[0], rhi = b.nodes[1];  // Bvh::bounds = nodes[0].aabb (bvh.rs:499-501)
-        const float* m = xf + 16ull * i;
-        float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
-        float hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        for (int c = 0; c < 8; ++c) {
-            float p[3];
-            xf_point_g(m, (c & 1) ? rhi.x : rlo.x, (c & 2) ? rhi.y : rlo.y, (c & 4) ? rhi.z : rlo.z, p);
-            for (int k = 0; k < 3; ++k) {
-                lo[k] = min_ni(lo[k], p[k]);
-                hi[k] = max_ni(hi[k], p[k]);
-            }
-        }
-        S.lx[i] = lo[0];
-        S.ly[i] = lo[1];
-        S.lz[i] = lo[2];
-        S.hx[i] = hi[0];
-        S.hy[i] = hi[1];
-        S.hz[i] = hi[2];
-        S.node[i] = 1 + i;  // leaves at 1..nobj (tlas.rs:210-218)
-        store_tlas_node(tlas_out, 1u + (uint32_t)i, Box6{lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]}, 0u, (uint32_t)i);
+        const Box6 o = object_bounds(blas_table[obj_blas[i]], xf + 16ull * i);
+        S.lx[i] = o.lx;
+        S.ly[i] = o.ly;
+        S.lz[i] = o.lz;
+        S.hx[i] = o.hx;
+        S.hy[i] = o.hy;
+        S.hz[i] = o.hz;
+        S.node[i] = 1 + i;
+        store_tlas_node(tlas_out, 1u + (uint32_t)i, o, 0u, (uint32_t)i);
     }
     __syncthreads();
     int count = n, used = 1 + n, a = 0;
     uint32_t err = 0;
     uint64_t steps = 0;
     const uint64_t max_steps = 4ull * nobj * nobj + 64;
-    if (n > (int)kTlasCachedObjects) {
-        // the reference's walk as written: every find_best_match a full scan by the block (no cache:
-        // with many objects the merged clusters become the cached best of many positions, whose
-        // rescans after each merge grow as n^2 per merge)
-        auto best = [&](int p) {
-            if (tid == 0) s_key_a = kNoKey;
-            __syncthreads();
-            const int chunk = (count + nwarps - 1) / nwarps;
-            const int r0 = warp * chunk, r1 = min(count, r0 + chunk);
-            if (r0 < r1) {
-                const unsigned long long k = warp_best_key(S, p, r0, r1);
-                if (lane == 0 && k != kNoKey) atomicMin(&s_key_a, k);
+    auto best = [&](int p) {
+        if (tid == 0) s_key = kNoKey;
+        __syncthreads();
+        const int chunk = (count + nwarps - 1) / nwarps;
+        const int r0 = warp * chunk, r1 = min(count, r0 + chunk);
+        if (r0 < r1) {
+            const Box6 P = load_box(S, p);
+            unsigned long long k = kNoKey;
+            for (int r = r0 + lane; r < r1; r += 32) {
+                if (r == p) continue;
+                const unsigned long long kr = sa_key(P, load_box(S, r), r);
+                k = kr < k ? kr : k;
             }
-            __syncthreads();
-            const int r = key_pos(s_key_a);
-            __syncthreads();
-            return r;
-        };
-        int b = best(0);
-        while (count > 1) {
-            if (b < 0 || ++steps > max_steps) {
-                err = 1;
-                break;
-            }
-            const int c = best(b);
-            if (a != c) {
-                a = b;
-                b = c;
-                continue;
-            }
-            if (warp == 0) tlas_merge(S, n, tlas_out, a, b, count - 1, used, lane);
-            count -= 1;
-            used += 1;
-            __syncthreads();
-            b = best(a);
+            k = warp_min_key(k);
+            if (lane == 0 && k != kNoKey) atomicMin(&s_key, k);
         }
         __syncthreads();
-        if (tid == 0) {
-            if (err == 0) {
-                const uint32_t r = (uint32_t)S.node[a];
-                const float4 r0 = tlas_out[2ull * r], r1 = tlas_out[2ull * r + 1];
-                tlas_out[0] = r0;
-                tlas_out[1] = r1;
-            }
-            status[0] = (uint32_t)used;
-            status[1] = err;
-        }
-        return;
-    }
-    for (int p = warp; p < n; p += nwarps) {
-        const unsigned long long k = warp_best_key(S, p, 0, n);
-        if (lane == 0) S.key[p] = k;
-    }
-    __syncthreads();
-
-    int b = key_pos(S.key[0]);
+        const int r = key_pos(s_key);
+        __syncthreads();
+        return r;
+    };
+    int b = best(0);
     while (count > 1) {
         if (b < 0 || ++steps > max_steps) {
             err = 1;
             break;
         }
-        const int c = key_pos(S.key[b]);
+        const int c = best(b);
         if (a != c) {
             a = b;
             b = c;
             continue;
         }
-        const int last = count - 1;
-        // Between the previous merge's last barrier and here the threads only read keys, so
-        // warp 0 may rewrite the boxes and the node list right away.
-        if (warp == 0) {
-            tlas_merge(S, n, tlas_out, a, b, last, used, lane);
-            if (lane == 6) s_ninval = 0;  // last read before the previous merge's final barrier
-        }
-        count = last;
+        if (warp == 0) tlas_merge(S, n, tlas_out, a, b, count - 1, used, lane);
+        count -= 1;
         used += 1;
         __syncthreads();
-        // s_key_a was read for the previous walk step by every thread before the barrier above
-        if (tid == 0) s_key_a = kNoKey;
-        for (int p = tid; p < count; p += (int)blockDim.x) {
-            unsigned long long k = S.key[p];
-            const int q = key_pos(k);
-            if (p == a || p == b || q == a || q == b || q == last) {
-                S.key[p] = kNoKey;
-                S.inval[atomicAdd(&s_ninval, 1)] = p;
-                continue;
-            }
-            const Box6 P = load_box(S, p);
-            if (a < count) {
-                const unsigned long long ka = sa_key(P, S, a);
-                k = ka < k ? ka : k;
-            }
-            if (b < count) {
-                const unsigned long long kb = sa_key(P, S, b);
-                k = kb < k ? kb : k;
-            }
-            S.key[p] = k;
-        }
-        __syncthreads();
-        // full rescans (and position a's stale entry if a left the list): every target split into
-        // slices over the warps, slices combined with atomicMin
-        const int ninval = s_ninval;
-        const int ntarget = ninval + (a >= count ? 1 : 0);
-        if (ntarget > 0) {
-            const int slices = max(1, nwarps / ntarget);
-            const int chunk = (count + slices - 1) / slices;
-            for (int item = warp; item < ntarget * slices; item += nwarps) {
-                const int j = item / slices, sl = item - j * slices;
-                const int p = j < ninval ? S.inval[j] : a;
-                const int r0 = sl * chunk, r1 = min(count, r0 + chunk);
-                const unsigned long long k = warp_best_key(S, p, r0, r1);
-                if (lane == 0 && k != kNoKey) atomicMin(j < ninval ? &S.key[p] : &s_key_a, k);
-            }
-        }
-        __syncthreads();
-        b = key_pos(a < count ? S.key[a] : s_key_a);
+        b = best(a);
     }
     __syncthreads();  // the inner nodes written by warp 0's lanes are visible to thread 0
     if (tid == 0) {
@@ -1210,21 +1223,38 @@ cudaError_t launch_refit(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-size_t tlas_smem_bytes(uint32_t nobj) { return (8ull + 8ull * sizeof(float)) * nobj; }
+size_t tlas_work_bytes(uint32_t nobj) { return 7ull * sizeof(float) * nobj; }
+
+template <int B, int K>
+static cudaError_t tlas_rebuild_block(bvhgpu_ctx* ctx, DeviceScene& sc, cudaStream_t s) {
+    const size_t smem = 32ull * sc.nobjects;
+    if (smem > 48u * 1024u) {
+        const cudaError_t e = cudaFuncSetAttribute(k_tlas_rebuild<B, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * B * K);
+        if (e != cudaSuccess) return e;
+    }
+    k_tlas_rebuild<B, K><<<1, B, smem, s>>>(static_cast<const GBlas*>(sc.blas_table), sc.obj_blas, sc.xf, sc.nobjects,
+                                            sc.tlas, ctx->d_scratch + 8);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_tlas_rebuild(bvhgpu_ctx* ctx, DeviceScene& sc, cudaStream_t s) {
-    auto* gwork = static_cast<unsigned long long*>(sc.tlas_work);
-    const size_t smem = gwork != nullptr ? 0 : tlas_smem_bytes(sc.nobjects);
-    static bool attr_set = false;  // set outside graph capture: the first rebuild is scene_create's
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_tlas_rebuild, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)tlas_smem_bytes(kTlasSharedObjects));
-        attr_set = true;
-    }
     LaunchScope scope(ctx, BVHGPU_K_TLAS_BUILD, s);
-    k_tlas_rebuild<<<1, kTlasThreads, smem, s>>>(static_cast<const GBlas*>(sc.blas_table), sc.obj_blas, sc.xf,
-                                                  sc.nobjects, sc.tlas, ctx->d_scratch + 8, gwork);
     g_launches++;
+    const uint32_t n = sc.nobjects;
+    // The fewest threads that hold the list in 2, 4 or 8 clusters each: fewer warps make the barrier
+    // and the reductions of a scan shorter, more than 8 clusters a thread make the scan itself
+    // longer.  In us, at 256 objects: 32 x 8 295, 64 x 4 218, 128 x 2 184, 256 x 1 197 (every find_best_match
+    // as a scan of global memory 703; the block of 512 that cached each position's best 524); at 512: 128 x 4 433,
+    // 256 x 2 589, 512 x 1 805; at 1,000: 128 x 8 1,158, 256 x 4 1,124, 512 x 2 1,309, 1024 x 1 1,583 (scans of shared
+    // memory 2,913); at 4,096: 256 x 16 11,540, 512 x 8 11,590, 1024 x 4 12,980 (19,530).
+    if (n <= 256u) return tlas_rebuild_block<128, 2>(ctx, sc, s);
+    if (n <= 512u) return tlas_rebuild_block<128, 4>(ctx, sc, s);
+    if (n <= 1024u) return tlas_rebuild_block<256, 4>(ctx, sc, s);
+    if (n <= 2048u) return tlas_rebuild_block<256, 8>(ctx, sc, s);
+    static_assert(kTlasBlockObjects == 512u * 8u, "the largest block's list");
+    if (n <= kTlasBlockObjects) return tlas_rebuild_block<512, 8>(ctx, sc, s);
+    k_tlas_rebuild_large<<<1, kTlasThreads, 0, s>>>(static_cast<const GBlas*>(sc.blas_table), sc.obj_blas, sc.xf, n,
+                                                    sc.tlas, ctx->d_scratch + 8, static_cast<float*>(sc.tlas_work));
     return cudaGetLastError();
 }
 
