@@ -127,10 +127,11 @@ inline bvhgpu_tune_config default_config(int kernel) {
     const bool single = kernel == BVHGPU_K_TRACE_BLAS || kernel == BVHGPU_K_TRACE_SCENE;
     return bvhgpu_tune_config{128u, 5u, 256u, 16u, single ? 1u : 8u, 2000u};
 }
+// The default config, up to a margin limit at or above the tuner's largest candidate.
 inline bool default_tune(const bvhgpu_tune_config& c, int kernel) {
     const bvhgpu_tune_config d = default_config(kernel);
     return c.block == d.block && c.min_blocks == d.min_blocks && c.stack == d.stack && c.big_leaf == d.big_leaf &&
-           c.refill == d.refill && c.hidden == d.hidden;
+           c.refill == d.refill && c.hidden >= 1000u;
 }
 
 struct ProfileRec {

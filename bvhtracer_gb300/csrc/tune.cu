@@ -174,6 +174,11 @@ int bvhgpu_autotune(bvhgpu_ctx* ctx, const bvhgpu_tune_job* job, uint32_t reps, 
     };
     bvhgpu_tune_config cur = ctx->tune[j.kernel];
     if (!valid_config(cur)) cur = bvhgpu_tune_config{128u, 5u, 256u, 16u, 8u, 500u};
+    // start inside the search space: the margin limit moves to the nearest candidate
+    uint32_t hd = kHiddenValues[0];
+    for (uint32_t h : kHiddenValues)
+        if ((h > cur.hidden ? h - cur.hidden : cur.hidden - h) < (hd > cur.hidden ? hd - cur.hidden : cur.hidden - hd)) hd = h;
+    cur.hidden = hd;
     float cur_ms = time_of(cur);
     auto consider = [&](const bvhgpu_tune_config& c) {
         const float ms = time_of(c);

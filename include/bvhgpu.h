@@ -470,7 +470,8 @@ typedef struct bvhgpu_tune_config {
 } bvhgpu_tune_config;
 /* Defaults (the tuner's picks on GB300): block 128, min_blocks 5, stack 256, big_leaf 16, refill 8,
  * hidden 2000; for the single-ray kernels (TRACE_BLAS, TRACE_SCENE) refill 1.  While TRACE_BLAS has its
- * default config, launches of few rays run one warp per ray instead (same hits). */
+ * default config (hidden may be any value from 1000 on), launches of few rays run one warp per ray
+ * instead (same hits). */
 int bvhgpu_tune_get(bvhgpu_ctx* ctx, int kernel, bvhgpu_tune_config* out);
 /* BVHGPU_ERR_INVALID_ARG for a kernel that is not tunable or a shape / stack not compiled. */
 int bvhgpu_tune_set(bvhgpu_ctx* ctx, int kernel, const bvhgpu_tune_config* cfg);
@@ -498,8 +499,8 @@ typedef struct bvhgpu_tune_job {
     const bvhgpu_batch_item* items;
     uint32_t nitems;
 } bvhgpu_tune_job;
-/* Times the job under candidate configs -- a coordinate search from the current config over
- * launch shape, stack, big_leaf, refill and hidden, two sweeps; each candidate runs once untimed, then
+/* Times the job under candidate configs -- a coordinate search from the current config (its
+ * hidden moved to the nearest candidate) over launch shape, stack, big_leaf, refill and hidden, two sweeps; each candidate runs once untimed, then
  * `reps` times bracketed by events on the context's stream (median kept) -- stores the fastest
  * in the context and returns it with its ms per call (either pointer may be NULL).  The job's
  * outputs are overwritten.  Synchronous; not allowed during graph capture. */

@@ -97,7 +97,7 @@ def test_default_and_set_configs_agree(ctx):
     a = blas.intersect(rays)
     saved = ctx.tune_get(bt.K_TRACE_BLAS)
     try:
-        ctx.tune_set(bt.K_TRACE_BLAS, hidden=1000)  # a set config: the one-thread kernel
+        ctx.tune_set(bt.K_TRACE_BLAS, hidden=500)  # a set config: the one-thread kernel
         assert blas.intersect(rays).tobytes() == a.tobytes()
     finally:
         ctx.tune_set(bt.K_TRACE_BLAS, **saved)
