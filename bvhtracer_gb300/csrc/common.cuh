@@ -84,16 +84,22 @@ constexpr uint32_t kConeMask = 0x0FFFFFFFu;
 constexpr uint32_t kWideShift = 28;  // hidden interior count: bits 28-29 = children - 1 (2..4 children)
 constexpr uint32_t kAnyCone = 0xFFFFFFFFu;  // TravT::lcone: the margins hold in the whole hidden tree
 // Below this root-cone margin a ray keeps the root cone's margins in the whole hidden tree (the
-// finer cones would cost more to evaluate than they save).
-constexpr float kConeSwitchDuv = 0.05f;
+// finer cones would cost more to evaluate than they save).  Measured at 0.5 | 0.05 (where it stood
+// with wider margins): soup frame 331 | 453 us, animated instanced frame 1,529 | 1,716, 512 x 512
+// Lambertian gradient 605 | 644, uneven batch 3,272 | 3,376; never switching: the same frames, but a
+// scene in large units (a sphere of radius 10 seen from 30) needs the finer cones.
+constexpr float kConeSwitchDuv = 0.5f;
 
 // Interior: a reference branch (count 0) or a hidden one (kHiddenInterior | cone).
 __host__ __device__ __forceinline__ bool node_interior(uint32_t cnt) { return cnt == 0u || (cnt >> 30) == 1u; }
 __host__ __device__ __forceinline__ uint32_t hidden_table_u2(uint32_t ntris) { return (ntris + 1u) & ~1u; }
 // Reference leaves with at least this many triangles get a hidden tree, whose leaves hold at most
-// kHiddenLeafTris triangles (two packed pairs).
+// kHiddenLeafTris triangles (four packed pairs).  At 2 | 4 | 6 | 8 | 12 triangles, in us: full-HD frame with
+// bounces 764 | 790 | 765 | 786 | 823, soup frame 593 | 331 | 308 | 287 | 275, uneven batch 3,825 | 3,272 |
+// 2,848 | 2,785 | 2,638, Lambertian gradient 762 | 605 | 543 | 538 | 520, animated instanced frame 1,678 | 1,529 |
+// 1,538 | 1,548 | 1,583.
 constexpr uint32_t kHiddenMinLeaf = 16;
-constexpr uint32_t kHiddenLeafTris = 4;
+constexpr uint32_t kHiddenLeafTris = 8;
 static_assert(kHiddenMinLeaf > kHiddenLeafTris, "a hidden root is an interior node");
 
 __host__ __device__ __forceinline__ uint32_t pairs_in_order(uint32_t ntris) { return (ntris + 1u) / 2u; }

@@ -80,8 +80,8 @@ namespace bvhgpu {
 
 constexpr float kCullUnit = 5.9604645e-8f;  // u0 = 2^-24
 // A barycentric margin Du + Dv below which the bound from |det| >= 1e-4 is used as it is: the cone
-// would cost more to evaluate than its narrower margin saves.
-constexpr float kNarrowDuv = 0.05f;
+// would cost more to evaluate than its narrower margin saves (soup frame 453 us at 0.05, 399 at 0.5).
+constexpr float kNarrowDuv = 0.5f;
 constexpr float kCullHuge = 1e15f;
 
 BVHGPU_HD float cull_fmax(float a, float b) { return a > b ? a : b; }

@@ -111,6 +111,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace_blas(GBlas b, const float
 constexpr uint32_t kWideStack = 256;    // pending reference nodes, as the largest stack variant
 constexpr uint32_t kWideNodes = 224;    // pending hidden nodes; fuller: the leaf is tested in order
 constexpr uint32_t kWideLeaves = 96;    // live hidden leaves waiting to be tested
+constexpr uint32_t kLeafPairs = kHiddenLeafTris / 2u;    // pairs of a hidden leaf, at most
+constexpr uint32_t kLeavesPerRound = 32u / kLeafPairs;  // hidden leaves tested at once, one pair per lane
 constexpr int kWideWarps = 2;           // warps (rays) per block
 // Leaves of at most this many triangles are tested in order (8 rounds of 64).  4,000 camera rays
 // against a 4,096-triangle soup / a 20,480-triangle sphere: 13 / 15 us at 256, 512 and 1,024, 19 / 15
@@ -186,17 +188,17 @@ __device__ __forceinline__ bool wide_hidden(const GBlas& g, uint2 root, LeafCull
             nl += (uint32_t)__popc(ml);
             nn += (uint32_t)__popc(mn);
             __syncwarp();
-            if (nn && nl < 16u) continue;
+            if (nn && nl < kLeavesPerRound) continue;
         }
-        // the newest up to 16 live leaves, one pair per lane (a hidden leaf has one or two)
-        const uint32_t take = min(nl, 16u);
+        // the newest live leaves, one pair per lane
+        const uint32_t take = min(nl, kLeavesPerRound);
         if (take == 0u) continue;
         nl -= take;
-        const uint32_t slot = lane >> 1;
+        const uint32_t slot = lane / kLeafPairs, q = lane % kLeafPairs;
         if (slot < take) {
             const uint2 e = sm.leaves[nl + slot];
-            if ((lane & 1u) < (e.x & ~kHiddenLeaf)) {
-                const uint32_t p = e.y + (lane & 1u);
+            if (q < (e.x & ~kHiddenLeaf)) {
+                const uint32_t p = e.y + q;
                 const uint2 idx = __ldg(hidx + p);
                 const PairData pd = load_pair(g.pairs + 5ull * p);
                 const PairHit h = ray_terms(pd, origin_terms(pd, OX, OY, OZ, Z), DX, DY, DZ, Z, idx.x != kMiss, idx.y != kMiss);
