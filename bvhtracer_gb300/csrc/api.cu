@@ -148,10 +148,8 @@ void free_blas(DeviceBlas& b) {
     cudaFree(b.leaf_keys);
     cudaFree(b.hx);
     cudaFree(b.cones);
-    cudaFree(b.hwork);
-    cudaFree(b.hchunks);
-    cudaFree(b.hchunk0);
-    cudaFree(b.hpart);
+    cudaFree(b.hup);
+    cudaFree(b.hagg);
     cudaFree(b.harrivals);
     cudaFree(b.normals);
     cudaFree(b.tex_coords);
@@ -259,10 +257,7 @@ struct HiddenPlan {
     std::vector<float> nodes;  // 8 floats per hidden node (boxes 0 until refreshed)
     std::vector<uint2> table;  // per triangle index, rounded up to even (empty: no hidden tree)
     std::vector<uint2> slots;  // per hidden pair
-    std::vector<uint4> work;   // per hidden node (box), then per cone
-    std::vector<uint2> chunks;    // {group, first pair}: each group in kRefreshChunk-pair chunks
-    std::vector<uint32_t> chunk0;  // first chunk of each group, then the total
-    uint32_t nbox_chunks = 0;      // chunks of the node groups (they come first)
+    std::vector<uint4> up;     // per hidden node: sibling block, siblings, parent, the parent's cone
     uint32_t nhid = 0, nhp = 0, ncones = 0, depth = 0;
 };
 
@@ -348,11 +343,10 @@ void plan_hidden(const bvhgpu_node* nodes, uint32_t nodes_used, const std::vecto
     const uint32_t P0 = pairs_in_order(ntris);
     std::vector<uint32_t> ids;
     std::vector<SahTri> info;
-    std::vector<uint4> cones;  // cone work: {first pair, end pair, ~0, cone}
     // (first, count) of the subtree over ids[a, b) at `depth` (4-wide levels) below the hidden
     // root; its pairs are allocated contiguously.  An interior node gets its children from two
     // levels of binary SAH splits (2 to 4 ranges); nodes below the root get their own cone.
-    auto make = [&](auto&& self, uint32_t a, uint32_t b, uint32_t depth, uint32_t gov) -> uint2 {
+    auto make = [&](auto&& self, uint32_t a, uint32_t b, uint32_t depth, uint32_t gov, uint32_t me) -> uint2 {
         hp.depth = std::max(hp.depth, depth);
         if (b - a <= kHiddenLeafTris) {
             const uint32_t np = (b - a + 1) / 2;
@@ -364,9 +358,7 @@ void plan_hidden(const bvhgpu_node* nodes, uint32_t nodes_used, const std::vecto
             hp.nhp += np;
             return make_uint2(p0, kHiddenLeaf | np);
         }
-        const uint32_t pa = P0 + hp.nhp;
-        const uint32_t own = depth >= 1 ? hp.ncones++ : kNoRefresh;
-        if (own != kNoRefresh) gov = own;
+        if (depth >= 1) gov = hp.ncones++;
         // SAH down to 32 binary levels, then halves (a balanced rest keeps the stack need bounded)
         auto split = [&](uint32_t x, uint32_t y) {
             return 2 * depth < 32 ? sah_split(ids, info, x, y) : x + (y - x) / 2;
@@ -383,16 +375,13 @@ void plan_hidden(const bvhgpu_node* nodes, uint32_t nodes_used, const std::vecto
         const uint32_t li = hp.nhid;
         hp.nhid += k;
         hp.nodes.resize(8ull * hp.nhid, 0.0f);
-        hp.work.resize(hp.nhid);
+        hp.up.resize(hp.nhid, make_uint4(li, k, me, gov));
         for (uint32_t c = 0; c < k; ++c) {
-            const uint32_t pc = P0 + hp.nhp;
-            const uint2 meta = self(self, ranges[c], ranges[c + 1], depth + 1, gov);
+            const uint2 meta = self(self, ranges[c], ranges[c + 1], depth + 1, gov, li + c);
             float* o = &hp.nodes[8ull * (li + c)];
             std::memcpy(&o[3], &meta.x, 4);
             std::memcpy(&o[7], &meta.y, 4);
-            hp.work[li + c] = make_uint4(pc, P0 + hp.nhp, nodes_used + li + c, kNoRefresh);
         }
-        if (own != kNoRefresh) cones.push_back(make_uint4(pa, P0 + hp.nhp, kNoRefresh, own));
         return make_uint2(nodes_used + li, kHiddenInterior | ((k - 1) << kWideShift) | gov);
     };
     info.resize(ntris);
@@ -412,19 +401,9 @@ void plan_hidden(const bvhgpu_node* nodes, uint32_t nodes_used, const std::vecto
             }
             ids[k] = t;
         }
-        const uint32_t pa = P0 + hp.nhp;
         const uint32_t root_cone = hp.ncones++;
-        const uint2 root = make(make, 0, n.primitive_count, 0, root_cone);  // interior: >= 16 triangles
-        hp.table[n.left_first] = root;
-        cones.push_back(make_uint4(pa, P0 + hp.nhp, kNoRefresh, root_cone));
+        hp.table[n.left_first] = make(make, 0, n.primitive_count, 0, root_cone, kNoRefresh);  // interior: >= 16 triangles
     }
-    hp.work.insert(hp.work.end(), cones.begin(), cones.end());
-    for (uint32_t j = 0; j < hp.work.size(); ++j) {
-        hp.chunk0.push_back((uint32_t)hp.chunks.size());
-        for (uint32_t p = hp.work[j].x; p < hp.work[j].y; p += kRefreshChunk) hp.chunks.push_back(make_uint2(j, p));
-        if (hp.work[j].z != kNoRefresh) hp.nbox_chunks = (uint32_t)hp.chunks.size();  // node groups come first
-    }
-    hp.chunk0.push_back((uint32_t)hp.chunks.size());
 }
 
 }  // namespace
@@ -639,10 +618,6 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
     b.nhid = hp.nhid;
     b.nhp = hp.nhp;
     b.ncones = hp.ncones;
-    b.nwork = (uint32_t)hp.work.size();
-    b.nchunks = (uint32_t)hp.chunks.size();
-    b.nbox_chunks = hp.nbox_chunks;
-    const size_t part_bytes = std::max(sizeof(float2), sizeof(RefreshAgg)) * std::max<size_t>(1, hp.chunks.size());
     b.ref_depth = depth;
     b.depth = depth + 3 * hp.depth;  // a 4-wide hidden level can leave 3 children pending
     const uint64_t nodes_all = (uint64_t)nodes_used + hp.nhid + 1;  // + a spare record (4-wide reads)
@@ -666,11 +641,9 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
         (e = cudaMalloc(&d_tris9, 36ull * ntris)) != cudaSuccess ||
         (hx_bytes && (e = cudaMalloc(&b.hx, hx_bytes)) != cudaSuccess) ||
         (b.ncones && (e = cudaMalloc(&b.cones, 32ull * b.ncones)) != cudaSuccess) ||
-        (b.nwork && (e = cudaMalloc(&b.hwork, 16ull * b.nwork)) != cudaSuccess) ||
-        (b.nwork && (e = cudaMalloc(&b.hchunks, 8ull * b.nchunks)) != cudaSuccess) ||
-        (b.nwork && (e = cudaMalloc(&b.hchunk0, 4ull * (b.nwork + 1))) != cudaSuccess) ||
-        (b.nwork && (e = cudaMalloc(&b.hpart, part_bytes)) != cudaSuccess) ||
-        (b.nwork && (e = cudaMalloc(&b.harrivals, 4ull * b.nwork)) != cudaSuccess)) {
+        (b.nhid && (e = cudaMalloc(&b.hup, 16ull * b.nhid)) != cudaSuccess) ||
+        (b.nhid && (e = cudaMalloc(&b.hagg, 128ull * b.nhid)) != cudaSuccess) ||
+        (b.nhid && (e = cudaMalloc(&b.harrivals, 4ull * b.nhid)) != cudaSuccess)) {
         cleanup();
         return fail(ctx, BVHGPU_ERR_OUT_OF_MEMORY, "blas_upload: %s", cudaGetErrorString(e));
     }
@@ -688,10 +661,8 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
         (hx_bytes && (e = cudaMemcpy(b.hx, hp.table.data(), 8ull * hp.table.size(), cudaMemcpyHostToDevice)) != cudaSuccess) ||
         (hx_bytes && hp.nhp &&
          (e = cudaMemcpy(b.hx + hp.table.size(), hp.slots.data(), 8ull * hp.nhp, cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (b.nwork && (e = cudaMemcpy(b.hwork, hp.work.data(), 16ull * b.nwork, cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (b.nwork && (e = cudaMemcpy(b.hchunks, hp.chunks.data(), 8ull * b.nchunks, cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (b.nwork && (e = cudaMemcpy(b.hchunk0, hp.chunk0.data(), 4ull * (b.nwork + 1), cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (b.nwork && (e = cudaMemset(b.harrivals, 0, 4ull * b.nwork)) != cudaSuccess) ||
+        (b.nhid && (e = cudaMemcpy(b.hup, hp.up.data(), 16ull * b.nhid, cudaMemcpyHostToDevice)) != cudaSuccess) ||
+        (b.nhid && (e = cudaMemset(b.harrivals, 0, 4ull * b.nhid)) != cudaSuccess) ||
         (e = launch_write_tris(ctx, b, static_cast<const float*>(d_tris9), ctx->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) {
         cleanup();

@@ -333,6 +333,14 @@ __device__ __forceinline__ PairData load_pair(const ulonglong2* __restrict__ P) 
     return d;
 }
 
+// A hidden pair: idx gets the triangle indices of its two slots (kMiss: padding), which it keeps in the
+// words a pair in triangle order leaves unused.
+__device__ __forceinline__ PairData load_hidden_pair(const ulonglong2* __restrict__ P, uint2& idx) {
+    const ulonglong2 q4 = __ldg(P + 4);
+    idx = make_uint2((uint32_t)q4.y, (uint32_t)(q4.y >> 32));
+    return load_pair(P);
+}
+
 __device__ __forceinline__ OriginTerms origin_terms(const PairData& p, f2 OX, f2 OY, f2 OZ, f2 Z) {
     OriginTerms o;
     o.SX = f2_sub(OX, p.V0X);  // s = ray.origin - v0
@@ -437,15 +445,14 @@ struct LocalStack {
 // while the held hit came from the same reference leaf (`held`): the reference's in-order leaf loop
 // keeps the lowest index among equal t, and a hit from an earlier leaf keeps equal t out.
 __device__ __forceinline__ bool test_hidden_leaf(const GBlas& b, uint32_t first, uint32_t np, LaneRay& r, bool& held) {
-    const uint2* hidx = b.hx + hidden_table_u2(b.ntris) - pairs_in_order(b.ntris);
     const f2 OX = f2_pack(r.o.x, r.o.x), OY = f2_pack(r.o.y, r.o.y), OZ = f2_pack(r.o.z, r.o.z);
     const f2 DX = f2_pack(r.d.x, r.d.x), DY = f2_pack(r.d.y, r.d.y), DZ = f2_pack(r.d.z, r.d.z);
     const f2 Z = f2_neg_zero();
     bool better = false;
     for (uint32_t q = 0; q < np; ++q) {
         const uint32_t p = first + q;
-        const uint2 idx = __ldg(hidx + p);
-        const PairData pd = load_pair(b.pairs + 5ull * p);
+        uint2 idx;
+        const PairData pd = load_hidden_pair(b.pairs + 5ull * p, idx);
         const PairHit h = ray_terms(pd, origin_terms(pd, OX, OY, OZ, Z), DX, DY, DZ, Z, idx.x != kMiss, idx.y != kMiss);
         if (h.okA && (h.tA < r.ct || (h.tA == r.ct && held && idx.x < r.hp))) {
             r.ct = h.tA;
@@ -492,7 +499,7 @@ struct TraceCounts {
     uint32_t ref_nodes;    // reference interior nodes (each loads its two children, 64 B)
     uint32_t hid_boxes;    // hidden child boxes tested (32 B each; 2 to 4 per hidden interior node)
     uint32_t entries;      // hidden trees entered (the leaf's table entry, 32 B)
-    uint32_t hid_pairs;    // hidden pairs tested (80 B + 8 B slot indices)
+    uint32_t hid_pairs;    // hidden pairs tested (80 B)
     uint32_t lane_tris;    // triangles of small reference leaves tested by the lane (48 B)
     uint32_t coop_tris;    // triangles of big reference leaves tested by the warp (40 B a triangle)
     uint32_t cone_switches;  // margins recomputed for another cone (2 x 16 B cone record)

@@ -49,262 +49,228 @@ __global__ void k_write_tris(const float* __restrict__ tris9, uint32_t n, float4
 }
 
 // ---- hidden trees of the large leaves, refreshed after every triangle write -----------------
-// Hidden pairs: the triangles of each pair's two slots (membership fixed at upload) copied into the
-// packed layout.  Then one warp per hidden node and per cone record: the widened box of the
-// node's pairs, or for a cone record the bounds Q, B and the normal cone of its pairs (cull.cuh).
-__global__ void k_hidden_pairs(const float4* __restrict__ tris, const uint2* __restrict__ slots, uint32_t nhp,
-                               float* __restrict__ pairs) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nhp) return;
-    const uint2 idx = slots[j];
-    float* P = pairs + 20ull * j;
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t k = h ? idx.y : idx.x;
-        float4 v0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), e1 = v0, e2 = v0;
-        if (k != kMiss) {
-            v0 = tris[3ull * k];
-            e1 = tris[3ull * k + 1];
-            e2 = tris[3ull * k + 2];
-        }
-        const float c[9] = {v0.x, v0.y, v0.z, e1.x, e1.y, e1.z, e2.x, e2.y, e2.z};
-        for (int q = 0; q < 9; ++q) P[2 * q + h] = c[q];
-    }
-    P[18] = P[19] = 0.0f;
+// One launch, bottom-up: four lanes per hidden leaf (one per triangle pair; membership fixed at
+// upload) copy its triangles into the packed pairs and fold their bounds, edge sizes and normals;
+// then, as in the refit, the last child of a node to arrive (one counter per block of siblings,
+// reset by it) folds the siblings' aggregates in child order, writes the node's box and its cone
+// record, and climbs on.
+//  - Boxes, Q and B are minima and maxima of the triangles' own values: the same in any order.
+//  - A node's normal cone is built from its grandchildren's cones: the axis is the sum of the children's
+//    folded unit-normal sums (any axis is valid), and normals within phi_c of the line of a grandchild's
+//    axis are within theta_c + phi_c of the line of the node's axis (theta_c between the axes).
+// The quad of lanes climbs together, a child per lane.  What bounds it: the climb's dependent hops (a
+// counter, a fence and up to four 128-B records each).
+// Against two passes of every node over all its triangles (a warp per 256 pairs), which read each
+// pair twice per tree level, together with the triangle rewrite before it: 327,680-triangle mesh
+// 240 -> 87 us, 20,480 triangles 98 -> 57 us.  Building each cone from the children alone loosened the
+// roots (a sphere of radius 100 seen from 3,000: 1,126 -> 1,464 us, more leaves tested in order).
+struct HiddenAgg {
+    float lo[3], hi[3];  // raw bounds of v0, v0 + e1, v0 + e2
+    float e1m, e2m;      // largest |e1_i|, |e2_i|
+    float s[3];          // sum of the unit normals, each turned towards the others
+    float cphi, nmin;    // the cone around s: least |N . s| / (|N| |s|) (<= 0: none) and |N|
+    float finite;        // 1: every input was finite
+};
+constexpr float kNoEntry = 2.0f;  // cphi of a missing child
+
+// An aggregate is 8 float4: the node's own four, then its children's cones {s, cphi} (a leaf's first is
+// its own).
+__device__ __forceinline__ HiddenAgg load_agg(const float4* a) {
+    const float4 x = __ldcg(a), y = __ldcg(a + 1), z = __ldcg(a + 2), w = __ldcg(a + 3);
+    return HiddenAgg{{x.x, x.y, x.z}, {y.x, y.y, y.z}, x.w, y.w, {z.x, z.y, z.z}, z.w, w.x, w.y};
+}
+__device__ __forceinline__ HiddenAgg empty_agg() {
+    return HiddenAgg{{FLT_MAX, FLT_MAX, FLT_MAX}, {-FLT_MAX, -FLT_MAX, -FLT_MAX}, 0.0f, 0.0f, {0.0f, 0.0f, 0.0f}, kNoEntry,
+                     FLT_MAX, 1.0f};
 }
 
-// The refresh runs over chunks of at most kRefreshChunk pairs, one warp each, so that the large
-// groups near the hidden roots (up to ~10,000 pairs) are spread over many warps instead of
-// holding one warp each for the whole launch.  A group's chunks are consecutive; the last chunk of
-// a group to finish (arrival counter, reset by it) combines the group's partial results in chunk
-// order, so every result is deterministic.  Pass 1 (k_hidden_refresh_boxes): the raw box
-// aggregates of every group and, for cone groups, the sum of the sign-folded unit normals; a
-// node group writes its widened box, a cone group its axis and the bounds Q, B.  Pass 2
-// (k_hidden_refresh_cones, cone groups only): the cone's angle and the smallest normal, from the
-// axis.  Min / max are exact in any order: boxes and cone angles do not depend on the chunking;
-// the axis (a float sum) does, and any axis gives a valid cone.
-__device__ __forceinline__ void agg_init(RefreshAgg& g) {
-    for (int i = 0; i < 3; ++i) {
-        g.lo[i] = FLT_MAX;
-        g.hi[i] = -FLT_MAX;
-    }
-    g.e1m = g.e2m = 0.0f;
-    g.sx = g.sy = g.sz = 0.0f;
-    g.finite = true;
+// Adds b's normals to a's, turned towards them.
+__device__ __forceinline__ void fold_normals(float* a, const float* b) {
+    const float sg = (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]) < 0.0f ? -1.0f : 1.0f;
+    for (int i = 0; i < 3; ++i) a[i] += sg * b[i];
 }
 
-// Folds b into a: min / max of the bounds, sum of the normals.
-__device__ __forceinline__ void agg_fold(RefreshAgg& a, const RefreshAgg& b) {
+__device__ __forceinline__ void fold_bounds(HiddenAgg& a, const HiddenAgg& b) {
     for (int i = 0; i < 3; ++i) {
         a.lo[i] = fminf(a.lo[i], b.lo[i]);
         a.hi[i] = fmaxf(a.hi[i], b.hi[i]);
     }
     a.e1m = fmaxf(a.e1m, b.e1m);
     a.e2m = fmaxf(a.e2m, b.e2m);
-    a.sx += b.sx;
-    a.sy += b.sy;
-    a.sz += b.sz;
-    a.finite = a.finite && b.finite;
+    a.finite = fminf(a.finite, b.finite);
 }
 
-__device__ __forceinline__ RefreshAgg agg_shfl_xor(const RefreshAgg& g, int off) {
-    RefreshAgg o;
-    for (int i = 0; i < 3; ++i) {
-        o.lo[i] = __shfl_xor_sync(0xFFFFFFFFu, g.lo[i], off);
-        o.hi[i] = __shfl_xor_sync(0xFFFFFFFFu, g.hi[i], off);
-    }
-    o.e1m = __shfl_xor_sync(0xFFFFFFFFu, g.e1m, off);
-    o.e2m = __shfl_xor_sync(0xFFFFFFFFu, g.e2m, off);
-    o.sx = __shfl_xor_sync(0xFFFFFFFFu, g.sx, off);
-    o.sy = __shfl_xor_sync(0xFFFFFFFFu, g.sy, off);
-    o.sz = __shfl_xor_sync(0xFFFFFFFFu, g.sz, off);
-    o.finite = __shfl_xor_sync(0xFFFFFFFFu, g.finite ? 1 : 0, off) != 0;
-    return o;
-}
-
-// The warp's fold of every lane's aggregate (the same fixed tree on every lane).
-__device__ __forceinline__ void agg_warp(RefreshAgg& g) {
-    for (int off = 16; off > 0; off >>= 1) agg_fold(g, agg_shfl_xor(g, off));
-}
-
-// The first valid normal of a cone group in pair order (the sign reference of its folded normals).
-__device__ __forceinline__ float3 group_reference_normal(const float* __restrict__ pairs, const uint2* __restrict__ slots,
-                                                         uint32_t p0, uint32_t first, uint32_t end) {
-    float rx = 0.0f, ry = 0.0f, rz = 0.0f;
-    if ((threadIdx.x & 31u) == 0u) {
-        for (uint32_t p = first; p < end; ++p) {
-            const uint2 idx = slots[p - p0];
-            const float* P = pairs + 20ull * p;
-            bool found = false;
-            for (int h = 0; h < 2 && !found; ++h) {
-                if ((h ? idx.y : idx.x) == kMiss) continue;
-                const float a[3] = {P[6 + h], P[8 + h], P[10 + h]}, b[3] = {P[12 + h], P[14 + h], P[16 + h]};
-                rx = a[1] * b[2] - a[2] * b[1];
-                ry = a[2] * b[0] - a[0] * b[2];
-                rz = a[0] * b[1] - a[1] * b[0];
-                found = isfinite(rx) && isfinite(ry) && isfinite(rz) && (rx != 0.0f || ry != 0.0f || rz != 0.0f);
-            }
-            if (found) break;
+// The fold of the four lanes' aggregates, the same in all four (a lower lane's normals before a higher
+// one's); cphi is left alone.
+__device__ __forceinline__ void quad_fold(HiddenAgg& g, unsigned quad) {
+#pragma unroll
+    for (int off = 1; off <= 2; off <<= 1) {
+        HiddenAgg o;
+        for (int j = 0; j < 3; ++j) {
+            o.lo[j] = __shfl_xor_sync(quad, g.lo[j], off);
+            o.hi[j] = __shfl_xor_sync(quad, g.hi[j], off);
+            o.s[j] = __shfl_xor_sync(quad, g.s[j], off);
+        }
+        o.e1m = __shfl_xor_sync(quad, g.e1m, off);
+        o.e2m = __shfl_xor_sync(quad, g.e2m, off);
+        o.finite = __shfl_xor_sync(quad, g.finite, off);
+        g.nmin = fminf(g.nmin, __shfl_xor_sync(quad, g.nmin, off));
+        fold_bounds(g, o);
+        if (threadIdx.x & off) {
+            fold_normals(o.s, g.s);
+            for (int j = 0; j < 3; ++j) g.s[j] = o.s[j];
+        } else {
+            fold_normals(g.s, o.s);
         }
     }
-    return make_float3(__shfl_sync(0xFFFFFFFFu, rx, 0), __shfl_sync(0xFFFFFFFFu, ry, 0), __shfl_sync(0xFFFFFFFFu, rz, 0));
+}
+__device__ __forceinline__ float quad_min(float v, unsigned quad) {
+    v = fminf(v, __shfl_xor_sync(quad, v, 1));
+    return fminf(v, __shfl_xor_sync(quad, v, 2));
 }
 
-// Pass 1, one warp per chunk {group, first pair}.
-__global__ void k_hidden_refresh_boxes(const uint4* __restrict__ work, const uint2* __restrict__ chunks, uint32_t nchunks,
-                                       const uint32_t* __restrict__ chunk0, RefreshAgg* __restrict__ part,
-                                       uint32_t* __restrict__ arrivals, const float* __restrict__ pairs,
-                                       const uint2* __restrict__ slots, uint32_t p0, float4* __restrict__ nodes,
-                                       float4* __restrict__ cones) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31u;
-    if (w >= nchunks) return;  // whole warps leave together
-    const uint2 ch = chunks[w];
-    const uint4 job = work[ch.x];
-    const uint32_t end = min(ch.y + kRefreshChunk, job.y);
-    const bool cone = job.w != kNoRefresh;
-    RefreshAgg g;
-    agg_init(g);
-    for (uint32_t p = ch.y + lane; p < end; p += 32u) {
+// A lower bound of |cos| between normals within phi_c (cphi) of the line of axis s, and the line of axis a
+// (cos(theta + phi), rounded down as in cone_det_lo); <= 0 where it gives none.
+__device__ __forceinline__ float wider_cone(const float* a, const float* s, float cphi) {
+    const float u0 = kCullUnit;
+    if (!(cphi > 0.0f) || !(cphi <= 1.0f)) return -1.0f;
+    const float dot = a[0] * s[0] + a[1] * s[1] + a[2] * s[2];
+    const float err = 4.0f * u0 * (fabsf(a[0] * s[0]) + fabsf(a[1] * s[1]) + fabsf(a[2] * s[2]));
+    const float la = sqrtf(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]), ls = sqrtf(s[0] * s[0] + s[1] * s[1] + s[2] * s[2]);
+    float ct = (fabsf(dot) - err) / (la * ls * (1.0f + 8.0f * u0)) * (1.0f - 4.0f * u0);
+    if (!(ct > 0.0f)) return -1.0f;
+    ct = fminf(ct, 1.0f);
+    const float st = cone_sin(ct), sp = cone_sin(cphi);
+    const float c = (ct * cphi * (1.0f - 4.0f * u0) - st * sp * (1.0f + 4.0f * u0)) * (1.0f - 4.0f * u0);
+    return c > 0.0f ? c : -1.0f;
+}
+
+// up[i] of hidden node i (both counted from the first hidden node): {first node of its sibling block,
+// siblings, parent node (kNoRefresh: a hidden root), the parent's cone record}.
+__global__ void __launch_bounds__(256) k_hidden_refresh(const float4* __restrict__ tris, const uint2* __restrict__ slots,
+                                                        uint32_t p0, float4* __restrict__ pairs,
+                                                        float4* nodes, uint32_t nhid, const uint4* __restrict__ up,
+                                                        float4* agg, uint32_t* arrivals, float4* __restrict__ cones) {
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, q = threadIdx.x & 3u;
+    uint32_t first = 0u, count = 0u;
+    if (i < nhid) {
+        first = __float_as_uint(nodes[2ull * i].w);
+        count = __float_as_uint(nodes[2ull * i + 1].w);
+    }
+    const bool leaf = (count & kHiddenLeaf) != 0u;
+    HiddenAgg g = empty_agg();
+    float c[2][9];
+    bool have[2] = {false, false};
+    if (leaf && q < (count & ~kHiddenLeaf)) {
+        const uint32_t p = first + q;
         const uint2 idx = slots[p - p0];
-        const float* P = pairs + 20ull * p;
+#pragma unroll
         for (int h = 0; h < 2; ++h) {
-            if ((h ? idx.y : idx.x) == kMiss) continue;
-            for (int i = 0; i < 3; ++i) {
-                const float v = P[2 * i + h], a = P[2 * (3 + i) + h], b = P[2 * (6 + i) + h];
-                const float p1 = fadd(v, a), p2 = fadd(v, b);
-                g.finite = g.finite && isfinite(v) && isfinite(a) && isfinite(b) && isfinite(p1) && isfinite(p2);
-                g.lo[i] = fminf(g.lo[i], fminf(v, fminf(p1, p2)));
-                g.hi[i] = fmaxf(g.hi[i], fmaxf(v, fmaxf(p1, p2)));
+            const uint32_t k = h ? idx.y : idx.x;
+            have[h] = k != kMiss;
+            float4 v0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), e1 = v0, e2 = v0;
+            if (have[h]) {
+                v0 = tris[3ull * k];
+                e1 = tris[3ull * k + 1];
+                e2 = tris[3ull * k + 2];
+            }
+            const float t[9] = {v0.x, v0.y, v0.z, e1.x, e1.y, e1.z, e2.x, e2.y, e2.z};
+            for (int j = 0; j < 9; ++j) c[h][j] = t[j];
+        }
+        // the packed pair, its triangles' indices in the last two words
+        float4* P = pairs + 5ull * p;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) P[j] = make_float4(c[0][2 * j], c[1][2 * j], c[0][2 * j + 1], c[1][2 * j + 1]);
+        P[4] = make_float4(c[0][8], c[1][8], __uint_as_float(idx.x), __uint_as_float(idx.y));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!have[h]) continue;
+            bool fin = true;
+            for (int j = 0; j < 3; ++j) {
+                const float v = c[h][j], a = c[h][3 + j], b = c[h][6 + j], p1 = fadd(v, a), p2 = fadd(v, b);
+                fin = fin && isfinite(v) && isfinite(a) && isfinite(b) && isfinite(p1) && isfinite(p2);
+                g.lo[j] = fminf(g.lo[j], fminf(v, fminf(p1, p2)));
+                g.hi[j] = fmaxf(g.hi[j], fmaxf(v, fmaxf(p1, p2)));
                 g.e1m = fmaxf(g.e1m, fabsf(a));
                 g.e2m = fmaxf(g.e2m, fabsf(b));
             }
-        }
-    }
-    if (cone) {
-        // the sum of the unit normals, each turned towards the group's first one (any axis is
-        // valid; this one makes the cone narrow)
-        const float3 r = group_reference_normal(pairs, slots, p0, job.x, job.y);
-        for (uint32_t p = ch.y + lane; p < end; p += 32u) {
-            const uint2 idx = slots[p - p0];
-            const float* P = pairs + 20ull * p;
-            for (int h = 0; h < 2; ++h) {
-                if ((h ? idx.y : idx.x) == kMiss) continue;
-                const float a[3] = {P[6 + h], P[8 + h], P[10 + h]}, b[3] = {P[12 + h], P[14 + h], P[16 + h]};
-                const float nx = a[1] * b[2] - a[2] * b[1], ny = a[2] * b[0] - a[0] * b[2], nz = a[0] * b[1] - a[1] * b[0];
-                const float len = sqrtf(nx * nx + ny * ny + nz * nz);
-                if (!(len > 0.0f) || !isfinite(len)) continue;
-                const float sg = (nx * r.x + ny * r.y + nz * r.z) < 0.0f ? -1.0f : 1.0f;
-                g.sx += sg * nx / len;
-                g.sy += sg * ny / len;
-                g.sz += sg * nz / len;
+            if (!fin) g.finite = 0.0f;
+            const float* a = c[h] + 3;
+            const float* b = c[h] + 6;
+            float n[3] = {a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2], a[0] * b[1] - a[1] * b[0]};
+            const float len = sqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+            if (len > 0.0f && isfinite(len)) {
+                for (int j = 0; j < 3; ++j) n[j] /= len;
+                fold_normals(g.s, n);
             }
         }
     }
-    agg_warp(g);
-    const uint32_t c0 = chunk0[ch.x], nc = chunk0[ch.x + 1] - c0;
-    if (nc > 1) {
-        // the group's last chunk to arrive combines the partials in chunk order
-        bool last = false;
-        if (lane == 0u) {
-            part[w] = g;
-            __threadfence();
-            last = atomicAdd(arrivals + ch.x, 1u) == nc - 1u;
+    if (!leaf) return;  // whole quads leave together
+    const unsigned quad = 0xFu << (threadIdx.x & 28u);
+    quad_fold(g, quad);
+    g.nmin = FLT_MAX;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (!have[h]) continue;
+        float cl, nl;
+        cone_terms(c[h] + 3, c[h] + 6, g.s[0], g.s[1], g.s[2], cl, nl);
+        g.cphi = cl < g.cphi ? cl : (cl == cl ? g.cphi : -1.0f);  // NaN: no cone
+        g.nmin = nl < g.nmin ? nl : (nl == nl ? g.nmin : 0.0f);
+    }
+    g.cphi = quad_min(g.cphi, quad);
+    g.nmin = quad_min(g.nmin, quad);
+    float4 entry = make_float4(g.s[0], g.s[1], g.s[2], q == 0u ? g.cphi : kNoEntry);  // cone of the node's child q
+    uint32_t cur = i;
+    for (;;) {
+        const GroupSeal box = group_seal(g.lo, g.hi, g.e1m, g.e2m, g.finite != 0.0f);
+        if (q < 3u) {  // first and count stay
+            reinterpret_cast<float*>(nodes + 2ull * cur)[q] = box.lo[q];
+            reinterpret_cast<float*>(nodes + 2ull * cur + 1)[q] = box.hi[q];
         }
-        if (!__shfl_sync(0xFFFFFFFFu, last ? 1 : 0, 0)) return;
+        float4* a = agg + 8ull * cur;
+        __stcg(a + q, q == 0u   ? make_float4(g.lo[0], g.lo[1], g.lo[2], g.e1m)
+                      : q == 1u ? make_float4(g.hi[0], g.hi[1], g.hi[2], g.e2m)
+                      : q == 2u ? make_float4(g.s[0], g.s[1], g.s[2], g.cphi)
+                                : make_float4(g.nmin, g.finite, 0.0f, 0.0f));
+        __stcg(a + 4u + q, entry);
+        const uint4 u = up[cur];
         __threadfence();
-        agg_init(g);
-        for (uint32_t k = lane; k < nc; k += 32u) {
-            const RefreshAgg* q = part + c0 + k;
-            RefreshAgg o;
-            for (int i = 0; i < 3; ++i) {
-                o.lo[i] = __ldcg(&q->lo[i]);
-                o.hi[i] = __ldcg(&q->hi[i]);
+        __syncwarp(quad);
+        uint32_t arrived = 0u;
+        if (q == 0u) arrived = atomicAdd(arrivals + u.x, 1u);
+        arrived = __shfl_sync(quad, arrived, (int)(threadIdx.x & 28u));
+        if (arrived != u.y - 1u) return;        // a sibling is still to come
+        if (q == 0u) arrivals[u.x] = 0u;        // ready for the next refresh
+        __threadfence();
+        // lane q: child q and its children's cones
+        g = empty_agg();
+        float4 below[4];
+        const float4* ch = agg + 8ull * (u.x + q);
+        if (q < u.y) {
+            g = load_agg(ch);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) below[j] = __ldcg(ch + 4 + j);
+        }
+        entry = make_float4(g.s[0], g.s[1], g.s[2], g.cphi);
+        quad_fold(g, quad);
+        float cphi = kNoEntry;
+        if (q < u.y) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float s[3] = {below[j].x, below[j].y, below[j].z};
+                if (below[j].w != kNoEntry) cphi = fminf(cphi, wider_cone(g.s, s, below[j].w));
             }
-            o.e1m = __ldcg(&q->e1m);
-            o.e2m = __ldcg(&q->e2m);
-            o.sx = __ldcg(&q->sx);
-            o.sy = __ldcg(&q->sy);
-            o.sz = __ldcg(&q->sz);
-            o.finite = *reinterpret_cast<volatile const bool*>(&q->finite);
-            agg_fold(g, o);
         }
-        agg_warp(g);
-        if (lane == 0u) arrivals[ch.x] = 0u;  // ready for the next refresh
+        g.cphi = quad_min(cphi, quad);
+        const GroupSeal seal = group_seal(g.lo, g.hi, g.e1m, g.e2m, g.finite != 0.0f);
+        const bool ok = isfinite(g.s[0]) && isfinite(g.s[1]) && isfinite(g.s[2]) && g.cphi > 0.0f && g.cphi <= 1.0f &&
+                        g.nmin > 0.0f && g.nmin < FLT_MAX;
+        if (!ok) g.cphi = -1.0f;
+        if (q == 0u) cones[2ull * u.w] = make_float4(ok ? g.s[0] : 0.0f, ok ? g.s[1] : 0.0f, ok ? g.s[2] : 0.0f, g.cphi);
+        if (q == 1u) cones[2ull * u.w + 1] = make_float4(ok ? cone_sin(g.cphi) : 1.0f, ok ? g.nmin : 0.0f, seal.q, seal.b);
+        if (u.z == kNoRefresh) return;
+        cur = u.z;
     }
-    if (lane != 0u) return;
-    const GroupSeal s = group_seal(g.lo, g.hi, g.e1m, g.e2m, g.finite);
-    if (!cone) {  // a node's box
-        float4* N = nodes + 2ull * job.z;
-        N[0] = make_float4(s.lo[0], s.lo[1], s.lo[2], N[0].w);
-        N[1] = make_float4(s.hi[0], s.hi[1], s.hi[2], N[1].w);
-        return;
-    }
-    // the axis and the bounds Q, B, for pass 2
-    float4* C = cones + 2ull * job.w;
-    C[0] = make_float4(g.sx, g.sy, g.sz, 0.0f);
-    C[1] = make_float4(0.0f, 0.0f, s.q, s.b);
-}
-
-// Pass 2, one warp per chunk of a cone group: the cone of the normal lines around the axis.
-__global__ void k_hidden_refresh_cones(const uint4* __restrict__ work, const uint2* __restrict__ chunks,
-                                       uint32_t first_chunk, uint32_t nchunks, const uint32_t* __restrict__ chunk0,
-                                       float2* __restrict__ part, uint32_t* __restrict__ arrivals,
-                                       const float* __restrict__ pairs, const uint2* __restrict__ slots, uint32_t p0,
-                                       float4* __restrict__ cones) {
-    const uint32_t w = first_chunk + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const unsigned lane = threadIdx.x & 31u;
-    if (w >= nchunks) return;  // whole warps leave together
-    const uint2 ch = chunks[w];
-    const uint4 job = work[ch.x];
-    const uint32_t end = min(ch.y + kRefreshChunk, job.y);
-    float4* C = cones + 2ull * job.w;
-    const float4 ax = __ldcg(C);
-    float cmin = 2.0f, nmin = FLT_MAX;
-    for (uint32_t p = ch.y + lane; p < end; p += 32u) {
-        const uint2 idx = slots[p - p0];
-        const float* P = pairs + 20ull * p;
-        for (int h = 0; h < 2; ++h) {
-            if ((h ? idx.y : idx.x) == kMiss) continue;
-            const float a[3] = {P[6 + h], P[8 + h], P[10 + h]}, b[3] = {P[12 + h], P[14 + h], P[16 + h]};
-            float cl, nl;
-            cone_terms(a, b, ax.x, ax.y, ax.z, cl, nl);
-            cmin = cl < cmin ? cl : (cl == cl ? cmin : -1.0f);  // NaN: no cone
-            nmin = nl < nmin ? nl : (nl == nl ? nmin : 0.0f);
-        }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        cmin = fminf(cmin, __shfl_xor_sync(0xFFFFFFFFu, cmin, off));
-        nmin = fminf(nmin, __shfl_xor_sync(0xFFFFFFFFu, nmin, off));
-    }
-    const uint32_t c0 = chunk0[ch.x], nc = chunk0[ch.x + 1] - c0;
-    if (nc > 1) {
-        bool last = false;
-        if (lane == 0u) {
-            part[w] = make_float2(cmin, nmin);
-            __threadfence();
-            last = atomicAdd(arrivals + ch.x, 1u) == nc - 1u;
-        }
-        if (!__shfl_sync(0xFFFFFFFFu, last ? 1 : 0, 0)) return;
-        __threadfence();
-        cmin = 2.0f;
-        nmin = FLT_MAX;
-        for (uint32_t k = lane; k < nc; k += 32u) {
-            const float2 q = __ldcg(part + c0 + k);
-            cmin = fminf(cmin, q.x);
-            nmin = fminf(nmin, q.y);
-        }
-        for (int off = 16; off > 0; off >>= 1) {
-            cmin = fminf(cmin, __shfl_xor_sync(0xFFFFFFFFu, cmin, off));
-            nmin = fminf(nmin, __shfl_xor_sync(0xFFFFFFFFu, nmin, off));
-        }
-        if (lane == 0u) arrivals[ch.x] = 0u;
-    }
-    if (lane != 0u) return;
-    const float4 qb = __ldcg(C + 1);
-    const bool cone_ok = isfinite(ax.x) && isfinite(ax.y) && isfinite(ax.z) && cmin > 0.0f && cmin <= 1.0f &&
-                         nmin > 0.0f && nmin < FLT_MAX;
-    C[0] = make_float4(cone_ok ? ax.x : 0.0f, cone_ok ? ax.y : 0.0f, cone_ok ? ax.z : 0.0f, cone_ok ? cmin : -1.0f);
-    C[1] = make_float4(cone_ok ? cone_sin(cmin) : 1.0f, cone_ok ? nmin : 0.0f, qb.z, qb.w);
 }
 
 // ---- refit, parallel over triangles --------------------------------------------------------
@@ -1194,22 +1160,12 @@ cudaError_t launch_write_tris(bvhgpu_ctx* ctx, DeviceBlas& b, const float* d_tri
 }
 
 cudaError_t launch_hidden_refresh(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s) {
-    if (b.nwork == 0) return cudaSuccess;
+    if (b.nhid == 0) return cudaSuccess;
     LaunchScope scope(ctx, BVHGPU_K_OTHER, s);
-    const uint32_t p0 = pairs_in_order(b.ntris);
-    const uint2* slots = b.hx + hidden_table_u2(b.ntris);
-    float* pairs = reinterpret_cast<float*>(b.pairs);
-    k_hidden_pairs<<<grid_for(b.nhp, 256), 256, 0, s>>>(b.tris, slots, b.nhp, pairs + 20ull * p0);
-    k_hidden_refresh_boxes<<<grid_for(32u * b.nchunks, 128), 128, 0, s>>>(
-        b.hwork, b.hchunks, b.nchunks, b.hchunk0, static_cast<RefreshAgg*>(b.hpart), b.harrivals, pairs, slots, p0,
-        b.nodes, b.cones);
-    g_launches += 2;
-    if (b.nchunks > b.nbox_chunks) {
-        k_hidden_refresh_cones<<<grid_for(32u * (b.nchunks - b.nbox_chunks), 128), 128, 0, s>>>(
-            b.hwork, b.hchunks, b.nbox_chunks, b.nchunks, b.hchunk0, static_cast<float2*>(b.hpart), b.harrivals,
-            pairs, slots, p0, b.cones);
-        g_launches++;
-    }
+    k_hidden_refresh<<<grid_for(4u * b.nhid, 256), 256, 0, s>>>(
+        b.tris, b.hx + hidden_table_u2(b.ntris), pairs_in_order(b.ntris), reinterpret_cast<float4*>(b.pairs),
+        b.nodes + 2ull * b.nodes_used, b.nhid, b.hup, b.hagg, b.harrivals, b.cones);
+    g_launches++;
     return cudaGetLastError();
 }
 

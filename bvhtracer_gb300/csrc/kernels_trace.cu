@@ -154,7 +154,6 @@ __device__ __forceinline__ bool wide_hidden(const GBlas& g, uint2 root, LeafCull
                                             WideSmem& sm) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
-    const uint2* hidx = g.hx + hidden_table_u2(g.ntris) - pairs_in_order(g.ntris);
     const f2 OX = f2_pack(r.o.x, r.o.x), OY = f2_pack(r.o.y, r.o.y), OZ = f2_pack(r.o.z, r.o.z);
     const f2 DX = f2_pack(r.d.x, r.d.x), DY = f2_pack(r.d.y, r.d.y), DZ = f2_pack(r.d.z, r.d.z);
     const f2 Z = f2_neg_zero();
@@ -199,8 +198,8 @@ __device__ __forceinline__ bool wide_hidden(const GBlas& g, uint2 root, LeafCull
             const uint2 e = sm.leaves[nl + slot];
             if (q < (e.x & ~kHiddenLeaf)) {
                 const uint32_t p = e.y + q;
-                const uint2 idx = __ldg(hidx + p);
-                const PairData pd = load_pair(g.pairs + 5ull * p);
+                uint2 idx;
+                const PairData pd = load_hidden_pair(g.pairs + 5ull * p, idx);
                 const PairHit h = ray_terms(pd, origin_terms(pd, OX, OY, OZ, Z), DX, DY, DZ, Z, idx.x != kMiss, idx.y != kMiss);
                 if (h.okA && (h.tA < b.t || (h.tA == b.t && b.k != kMiss && idx.x < b.k))) {
                     b.t = h.tA;
