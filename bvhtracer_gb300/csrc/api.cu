@@ -245,167 +245,6 @@ void pack_nodes(const bvhgpu_node* nodes, uint32_t n, std::vector<float>& out) {
     }
 }
 
-// Hidden trees over the leaves with at least kHiddenMinLeaf triangles, built by binned SAH: a range
-// of triangles is split at the cheapest of 15 planes (16 bins of the centroids along the widest
-// centroid axis, cost = area x count of each side), in halves by index order when the centroids
-// coincide or below 32 binary levels, down to at most kHiddenLeafTris triangles stored as packed
-// pairs (a padding slot is all zero with index 0xFFFFFFFF).  Two levels of splits make one 4-wide
-// node.  Hidden nodes get indices from nodes_used on, a node's children consecutive, allocated
-// depth first; the boxes and the leaf bounds Q, B and normal cone are written
-// by the refresh kernels from `work`.  Only speed depends on the tree's shape.
-struct HiddenPlan {
-    std::vector<float> nodes;  // 8 floats per hidden node (boxes 0 until refreshed)
-    std::vector<uint2> table;  // per triangle index, rounded up to even (empty: no hidden tree)
-    std::vector<uint2> slots;  // per hidden pair
-    std::vector<uint4> up;     // per hidden node: sibling block, siblings, parent, the parent's cone
-    uint32_t nhid = 0, nhp = 0, ncones = 0, depth = 0;
-};
-
-struct SahTri {
-    float c[3], lo[3], hi[3];
-};
-
-inline float half_area(const float lo[3], const float hi[3]) {
-    const float e0 = hi[0] - lo[0], e1 = hi[1] - lo[1], e2 = hi[2] - lo[2];
-    return e0 * e1 + e1 * e2 + e2 * e0;
-}
-
-// Reorders ids[a, b) into two non-empty parts by the binned SAH; returns the split position.
-uint32_t sah_split(std::vector<uint32_t>& ids, const std::vector<SahTri>& info, uint32_t a, uint32_t b) {
-    const uint32_t mid = a + (b - a) / 2;
-    float cl[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, ch[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (uint32_t j = a; j < b; ++j)
-        for (int k = 0; k < 3; ++k) {
-            cl[k] = std::min(cl[k], info[ids[j]].c[k]);
-            ch[k] = std::max(ch[k], info[ids[j]].c[k]);
-        }
-    int ax = 0;
-    for (int k = 1; k < 3; ++k)
-        if (ch[k] - cl[k] > ch[ax] - cl[ax]) ax = k;
-    const float ext = ch[ax] - cl[ax];
-    if (!(ext > 0.0f) || !(ext < FLT_MAX)) return mid;
-    constexpr int kBins = 16;
-    auto bin_of = [&](uint32_t id) {
-        const float x = (info[id].c[ax] - cl[ax]) / ext * (float)kBins;
-        return x >= 0.0f ? std::min(kBins - 1, (int)x) : 0;  // NaN -> 0
-    };
-    uint32_t cnt[kBins] = {};
-    float blo[kBins][3], bhi[kBins][3];
-    for (int i = 0; i < kBins; ++i)
-        for (int k = 0; k < 3; ++k) {
-            blo[i][k] = FLT_MAX;
-            bhi[i][k] = -FLT_MAX;
-        }
-    for (uint32_t j = a; j < b; ++j) {
-        const int i = bin_of(ids[j]);
-        ++cnt[i];
-        for (int k = 0; k < 3; ++k) {
-            blo[i][k] = std::min(blo[i][k], info[ids[j]].lo[k]);
-            bhi[i][k] = std::max(bhi[i][k], info[ids[j]].hi[k]);
-        }
-    }
-    float right_cost[kBins] = {};
-    float rlo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, rhi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    uint32_t rn = 0;
-    for (int i = kBins - 1; i > 0; --i) {  // right side = bins i..15
-        rn += cnt[i];
-        for (int k = 0; k < 3; ++k) {
-            rlo[k] = std::min(rlo[k], blo[i][k]);
-            rhi[k] = std::max(rhi[k], bhi[i][k]);
-        }
-        right_cost[i] = rn ? half_area(rlo, rhi) * (float)rn : 0.0f;
-    }
-    float llo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, lhi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    uint32_t ln = 0;
-    float best = FLT_MAX;
-    int best_bin = -1;  // left side = bins 0..best_bin
-    for (int i = 0; i < kBins - 1; ++i) {
-        ln += cnt[i];
-        for (int k = 0; k < 3; ++k) {
-            llo[k] = std::min(llo[k], blo[i][k]);
-            lhi[k] = std::max(lhi[k], bhi[i][k]);
-        }
-        if (ln == 0 || ln == b - a) continue;
-        const float cost = half_area(llo, lhi) * (float)ln + right_cost[i + 1];
-        if (cost < best) {
-            best = cost;
-            best_bin = i;
-        }
-    }
-    if (best_bin < 0) return mid;
-    auto it = std::stable_partition(ids.begin() + a, ids.begin() + b,
-                                    [&](uint32_t id) { return bin_of(id) <= best_bin; });
-    return (uint32_t)(it - ids.begin());
-}
-
-void plan_hidden(const bvhgpu_node* nodes, uint32_t nodes_used, const std::vector<uint32_t>& leaves,
-                 const bvhgpu_triangle* tris, uint32_t ntris, HiddenPlan& hp) {
-    const uint32_t P0 = pairs_in_order(ntris);
-    std::vector<uint32_t> ids;
-    std::vector<SahTri> info;
-    // (first, count) of the subtree over ids[a, b) at `depth` (4-wide levels) below the hidden
-    // root; its pairs are allocated contiguously.  An interior node gets its children from two
-    // levels of binary SAH splits (2 to 4 ranges); nodes below the root get their own cone.
-    auto make = [&](auto&& self, uint32_t a, uint32_t b, uint32_t depth, uint32_t gov, uint32_t me) -> uint2 {
-        hp.depth = std::max(hp.depth, depth);
-        if (b - a <= kHiddenLeafTris) {
-            const uint32_t np = (b - a + 1) / 2;
-            const uint32_t p0 = P0 + hp.nhp;
-            for (uint32_t q = 0; q < np; ++q) {
-                const uint32_t s0 = a + 2 * q;
-                hp.slots.push_back(make_uint2(ids[s0], s0 + 1 < b ? ids[s0 + 1] : kMiss));
-            }
-            hp.nhp += np;
-            return make_uint2(p0, kHiddenLeaf | np);
-        }
-        if (depth >= 1) gov = hp.ncones++;
-        // SAH down to 32 binary levels, then halves (a balanced rest keeps the stack need bounded)
-        auto split = [&](uint32_t x, uint32_t y) {
-            return 2 * depth < 32 ? sah_split(ids, info, x, y) : x + (y - x) / 2;
-        };
-        uint32_t ranges[5];
-        uint32_t nr = 0;
-        const uint32_t m = split(a, b);
-        ranges[nr++] = a;
-        if (m - a > kHiddenLeafTris) ranges[nr++] = split(a, m);
-        ranges[nr++] = m;
-        if (b - m > kHiddenLeafTris) ranges[nr++] = split(m, b);
-        ranges[nr] = b;
-        const uint32_t k = nr;  // 2..4 children
-        const uint32_t li = hp.nhid;
-        hp.nhid += k;
-        hp.nodes.resize(8ull * hp.nhid, 0.0f);
-        hp.up.resize(hp.nhid, make_uint4(li, k, me, gov));
-        for (uint32_t c = 0; c < k; ++c) {
-            const uint2 meta = self(self, ranges[c], ranges[c + 1], depth + 1, gov, li + c);
-            float* o = &hp.nodes[8ull * (li + c)];
-            std::memcpy(&o[3], &meta.x, 4);
-            std::memcpy(&o[7], &meta.y, 4);
-        }
-        return make_uint2(nodes_used + li, kHiddenInterior | ((k - 1) << kWideShift) | gov);
-    };
-    info.resize(ntris);
-    for (uint32_t li : leaves) {
-        const bvhgpu_node& n = nodes[li];
-        if (n.primitive_count < kHiddenMinLeaf) continue;
-        if (hp.table.empty()) hp.table.assign(hidden_table_u2(ntris), make_uint2(0u, 0u));
-        ids.resize(n.primitive_count);
-        for (uint32_t k = 0; k < n.primitive_count; ++k) {
-            const uint32_t t = n.left_first + k;
-            const float* v = tris[t].vertices;
-            SahTri& s = info[t];
-            for (int a = 0; a < 3; ++a) {
-                s.c[a] = (v[a] + v[3 + a] + v[6 + a]) / 3.0f;
-                s.lo[a] = std::min(v[a], std::min(v[3 + a], v[6 + a]));
-                s.hi[a] = std::max(v[a], std::max(v[3 + a], v[6 + a]));
-            }
-            ids[k] = t;
-        }
-        const uint32_t root_cone = hp.ncones++;
-        hp.table[n.left_first] = make(make, 0, n.primitive_count, 0, root_cone, kNoRefresh);  // interior: >= 16 triangles
-    }
-}
-
 }  // namespace
 
 extern "C" {
@@ -613,8 +452,26 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
     std::vector<unsigned long long> key_init(6 * std::max<size_t>(1, leaves.size()), 0ull);
     for (size_t li = 0; li < key_init.size() / 6; ++li)
         for (int k = 0; k < 3; ++k) key_init[6 * li + k] = 0xFFFFFFFFFFFFFFFFull;
+    void* d_tris9 = nullptr;
     HiddenPlan hp;
-    plan_hidden(nodes, nodes_used, leaves, tris, ntris, hp);
+    cudaError_t e = cudaSuccess;
+    auto cleanup = [&]() {
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(d_tris9);
+        cudaFree(hp.work);
+        free_blas(b);
+    };
+    if ((e = cudaMalloc(&d_tris9, 36ull * ntris)) != cudaSuccess) {
+        cleanup();
+        return fail(ctx, BVHGPU_ERR_OUT_OF_MEMORY, "blas_upload: %s", cudaGetErrorString(e));
+    }
+    if ((e = cudaMemcpyAsync(d_tris9, tris, 36ull * ntris, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess ||
+        (e = plan_hidden(ctx, nodes, nodes_used, leaves, static_cast<const float*>(d_tris9), ntris, hp, ctx->stream)) !=
+            cudaSuccess) {
+        cleanup();
+        return e == cudaErrorMemoryAllocation ? fail(ctx, BVHGPU_ERR_OUT_OF_MEMORY, "blas_upload: %s", cudaGetErrorString(e))
+                                              : cuda_fail(ctx, e, "blas_upload");
+    }
     b.nhid = hp.nhid;
     b.nhp = hp.nhp;
     b.ncones = hp.ncones;
@@ -622,13 +479,7 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
     b.depth = depth + 3 * hp.depth;  // a 4-wide hidden level can leave 3 children pending
     const uint64_t nodes_all = (uint64_t)nodes_used + hp.nhid + 1;  // + a spare record (4-wide reads)
     const uint64_t pairs_all = (uint64_t)pairs_in_order(ntris) + hp.nhp;
-    const uint64_t hx_bytes = hp.table.empty() ? 0 : 8ull * hidden_table_u2(ntris) + 8ull * std::max<uint32_t>(1, hp.nhp);
-    void* d_tris9 = nullptr;
-    cudaError_t e = cudaSuccess;
-    auto cleanup = [&]() {
-        cudaFree(d_tris9);
-        free_blas(b);
-    };
+    const uint64_t hx_bytes = hp.nhid == 0 ? 0 : 8ull * hp.table_u2 + 8ull * std::max<uint32_t>(1, hp.nhp);
     if ((e = cudaMalloc(&b.nodes, 32ull * nodes_all)) != cudaSuccess ||
         (e = cudaMalloc(&b.tris, 48ull * ntris)) != cudaSuccess ||
         (e = cudaMalloc(&b.verts, 48ull * ntris)) != cudaSuccess ||
@@ -638,7 +489,6 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
         (e = cudaMalloc(&b.counters, 4ull * nodes_used)) != cudaSuccess ||
         (e = cudaMalloc(&b.tri_leaf, 4ull * ntris)) != cudaSuccess ||
         (e = cudaMalloc(&b.leaf_keys, 48ull * std::max<size_t>(1, leaves.size()))) != cudaSuccess ||
-        (e = cudaMalloc(&d_tris9, 36ull * ntris)) != cudaSuccess ||
         (hx_bytes && (e = cudaMalloc(&b.hx, hx_bytes)) != cudaSuccess) ||
         (b.ncones && (e = cudaMalloc(&b.cones, 32ull * b.ncones)) != cudaSuccess) ||
         (b.nhid && (e = cudaMalloc(&b.hup, 16ull * b.nhid)) != cudaSuccess) ||
@@ -647,27 +497,23 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
         cleanup();
         return fail(ctx, BVHGPU_ERR_OUT_OF_MEMORY, "blas_upload: %s", cudaGetErrorString(e));
     }
-    if ((e = cudaMemcpy(b.nodes, packed.data(), 32ull * nodes_used, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(b.parent, parent.data(), 4ull * nodes_used, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(b.leaves, leaves.data(), 4ull * leaves.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemset(b.counters, 0, 4ull * nodes_used)) != cudaSuccess ||
-        (e = cudaMemset(b.nodes + 2ull * (nodes_all - 1), 0, 32)) != cudaSuccess ||
-        (e = cudaMemcpy(b.tri_leaf, tri_leaf.data(), 4ull * ntris, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(b.leaf_keys, key_init.data(), 8ull * key_init.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemset(b.pairs, 0, 80ull * pairs_all)) != cudaSuccess ||
-        (e = cudaMemcpy(d_tris9, tris, 36ull * ntris, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (hp.nhid && (e = cudaMemcpy(b.nodes + 2ull * nodes_used, hp.nodes.data(), 32ull * hp.nhid,
-                                    cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (hx_bytes && (e = cudaMemcpy(b.hx, hp.table.data(), 8ull * hp.table.size(), cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (hx_bytes && hp.nhp &&
-         (e = cudaMemcpy(b.hx + hp.table.size(), hp.slots.data(), 8ull * hp.nhp, cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (b.nhid && (e = cudaMemcpy(b.hup, hp.up.data(), 16ull * b.nhid, cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (b.nhid && (e = cudaMemset(b.harrivals, 0, 4ull * b.nhid)) != cudaSuccess) ||
-        (e = launch_write_tris(ctx, b, static_cast<const float*>(d_tris9), ctx->stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) {
+    const cudaStream_t st = ctx->stream;
+    if ((e = cudaMemcpyAsync(b.nodes, packed.data(), 32ull * nodes_used, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b.parent, parent.data(), 4ull * nodes_used, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b.leaves, leaves.data(), 4ull * leaves.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b.counters, 0, 4ull * nodes_used, st)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b.nodes + 2ull * (nodes_all - 1), 0, 32, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b.tri_leaf, tri_leaf.data(), 4ull * ntris, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b.leaf_keys, key_init.data(), 8ull * key_init.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b.pairs, 0, 80ull * pairs_all, st)) != cudaSuccess ||
+        (b.nhid && (e = cudaMemsetAsync(b.harrivals, 0, 4ull * b.nhid, st)) != cudaSuccess) ||
+        (e = finish_hidden(ctx, hp, b, st)) != cudaSuccess ||
+        (e = launch_write_tris(ctx, b, static_cast<const float*>(d_tris9), st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess) {
         cleanup();
         return cuda_fail(ctx, e, "blas_upload");
     }
+    cudaFree(hp.work);
     cudaFree(d_tris9);
     uint32_t id = ctx->next_blas++;
     ctx->blas[id] = b;

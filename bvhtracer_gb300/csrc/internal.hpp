@@ -51,6 +51,16 @@ struct DeviceBlas {
     uint32_t tex_w = 0, tex_h = 0;
 };
 
+// The hidden trees planned for a BLAS (plan_hidden.cu): sizes, and device arrays in `work` (owned by the
+// caller) that finish_hidden turns into the BLAS's records.
+struct HiddenPlan {
+    void* work = nullptr;
+    uint32_t nhid = 0, nhp = 0, ncones = 0, depth = 0, table_u2 = 0;
+    uint32_t *ids = nullptr, *pair_at = nullptr, *sums = nullptr;
+    uint2 *meta = nullptr, *range = nullptr, *table = nullptr;
+    uint4* up = nullptr;
+};
+
 // Per entry of a scene's BLAS table: what the normal / texture accumulators read of a model.
 struct ShadeEntry {
     const float* normals;
@@ -231,6 +241,14 @@ cudaError_t launch_render(bvhgpu_ctx* ctx, const DeviceBlas& b, const bvhgpu_cam
                           const float* acc_params, int shader, const float* shader_params, const float* d_normals,
                           const float* d_tex_coords, const uint8_t* d_texels, uint32_t tex_w, uint32_t tex_h,
                           uint8_t* d_rgba, cudaStream_t s);
+
+// ---- hidden-tree planning (plan_hidden.cu) ----------------------------------------------
+// Plans the hidden trees over the BLAS's large leaves from its triangles (device, 9 floats each);
+// synchronises the stream.  plan.work is allocated here, to be freed by the caller.
+cudaError_t plan_hidden(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes_used, const std::vector<uint32_t>& leaves,
+                        const float* d_tris9, uint32_t ntris, HiddenPlan& plan, cudaStream_t s);
+// Writes the plan into b.nodes, b.hx and b.hup (allocated for its sizes).
+cudaError_t finish_hidden(bvhgpu_ctx* ctx, const HiddenPlan& plan, DeviceBlas& b, cudaStream_t s);
 
 // ---- launchers (kernels_scene.cu) ------------------------------------------------------
 cudaError_t launch_write_tris(bvhgpu_ctx* ctx, DeviceBlas& b, const float* d_tris9, cudaStream_t s);
