@@ -960,6 +960,7 @@ int bvhgpu_scene_create(bvhgpu_ctx* ctx, const uint32_t* blas_ids, uint32_t nobj
     for (uint32_t i = 0; i < nobjects; ++i) {
         DeviceBlas* b = find_blas(ctx, blas_ids[i]);
         if (!b) return fail(ctx, BVHGPU_ERR_INVALID_ARG, "scene_create: unknown BLAS %u", blas_ids[i]);
+        sc.instanced_tris += b->ntris;
         auto it = std::find(sc.table_blas.begin(), sc.table_blas.end(), blas_ids[i]);
         if (it == sc.table_blas.end()) {
             sc.table_blas.push_back(blas_ids[i]);

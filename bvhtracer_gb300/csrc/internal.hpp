@@ -81,7 +81,7 @@ struct DeviceScene {
     float4* tlas = nullptr;    // 2 float4 per TLAS node (2*nobjects nodes)
     void* tlas_work = nullptr; // TLAS rebuild list (28 B per object) above kTlasBlockObjects objects
     uint32_t tlas_nodes_used = 0;
-    uint32_t tlas_depth_cap = 0;
+    uint64_t instanced_tris = 0;     // triangles of all objects
     uint32_t world = 0;              // bound physics world (0: none)
     uint32_t* body_of = nullptr;     // per object: body index or 0xFFFFFFFF
     float* transform_init = nullptr; // 16 per object

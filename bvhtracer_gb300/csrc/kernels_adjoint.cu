@@ -19,6 +19,7 @@
 #include "internal.hpp"
 #include "persistent.cuh"
 #include "variants.cuh"
+#include "wide.cuh"
 
 namespace bvhgpu {
 
@@ -254,6 +255,31 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_lambert_forward(GBlas b, const 
     }
 }
 
+// Forward pass of few rays: one warp per pixel (wide.cuh), without a schedule.
+__global__ void __launch_bounds__(32 * kWideWarps) k_lambert_forward_wide(GBlas b, const float4* __restrict__ rays, uint32_t n,
+                                                                          const uint32_t* __restrict__ faces,
+                                                                          const float* __restrict__ verts,
+                                                                          const float* __restrict__ vnormals, float3 light,
+                                                                          float* __restrict__ image, GHit* __restrict__ hits,
+                                                                          LeafPolicy pol, uint32_t* err) {
+    __shared__ WideSmem smem[kWideWarps];
+    const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
+    if (i >= n) return;
+    Deadline dl;
+    dl.start(err);
+    LaneRay r;
+    float3 o, d;
+    float t0;
+    load_ray(rays, i, o, d, t0);
+    init_lane_ray(r, o, d, t0);
+    wide_blas(b, r, pol, smem[threadIdx.x >> 5], dl, err);
+    if ((threadIdx.x & 31u) != 0u) return;
+    const bool hit = r.hit && r.ct < FLT_MAX;
+    store_hit(hits, i, hit, r.ct, r.hu, r.hv, r.hp, 0u);
+    Shade sh;
+    image[i] = hit ? shade(r.o, r.d, r.ct, r.hu, r.hv, faces, r.hp, verts, vnormals, light, sh) : 0.0f;
+}
+
 // Starts a scheduled forward pass over n rays: the next pass number (its parity alternates, also
 // across the counter's wrap), the previous pass's ray count (0, and an empty list, when that pass
 // stopped at a deadline), empty queues, and an empty list for the pass after it.
@@ -359,6 +385,13 @@ cudaError_t launch_lambert_forward(bvhgpu_ctx* ctx, DeviceMesh& m, const DeviceB
     // the launch shape, stack and leaf policy (big leaves, hidden-tree margin) of the plain trace
     // kernel's launch config, and its refill threshold
     const Variant v = resolve(ctx->tune[BVHGPU_K_TRACE_BLAS], b.depth);
+    if (n <= wide_rays(ctx, BVHGPU_K_TRACE_BLAS, b.ntris)) {
+        LaunchScope scope(ctx, BVHGPU_K_LAMBERT_FORWARD, s);
+        k_lambert_forward_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(
+            g, rays, n, m.faces, m.verts, m.vnormals, L, image, static_cast<GHit*>(hits), v.pol, ctx->d_err);
+        g_launches++;
+        return cudaGetLastError();
+    }
     uint32_t* queue = ctx->d_scratch + 5;
     cudaError_t e = cudaSuccess;
     // the long-ray schedule (ForwardSchedule): grown outside stream capture only; a captured pass

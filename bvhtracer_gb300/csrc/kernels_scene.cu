@@ -14,8 +14,10 @@
 
 #include "common.cuh"
 #include "internal.hpp"
+#include "persistent.cuh"
 #include "render.cuh"
 #include "variants.cuh"
+#include "wide.cuh"
 
 namespace bvhgpu {
 namespace {
@@ -726,6 +728,23 @@ struct SceneData {
     uint32_t tlas_nodes;
 };
 
+// SceneObject::intersect's ray: world ray (wo, wd) through the cached inverse m, 1/d' recomputed.
+__device__ __forceinline__ void to_model(const float* m, float3 wo, float3 wd, LaneRay& r) {
+    r.o.x = fadd(fadd(fadd(fmul(__ldg(m + 0), wo.x), fmul(__ldg(m + 4), wo.y)), fmul(__ldg(m + 8), wo.z)),
+                 fmul(__ldg(m + 12), 1.0f));
+    r.o.y = fadd(fadd(fadd(fmul(__ldg(m + 1), wo.x), fmul(__ldg(m + 5), wo.y)), fmul(__ldg(m + 9), wo.z)),
+                 fmul(__ldg(m + 13), 1.0f));
+    r.o.z = fadd(fadd(fadd(fmul(__ldg(m + 2), wo.x), fmul(__ldg(m + 6), wo.y)), fmul(__ldg(m + 10), wo.z)),
+                 fmul(__ldg(m + 14), 1.0f));
+    r.d.x = fadd(fadd(fadd(fmul(__ldg(m + 0), wd.x), fmul(__ldg(m + 4), wd.y)), fmul(__ldg(m + 8), wd.z)),
+                 fmul(__ldg(m + 12), 0.0f));
+    r.d.y = fadd(fadd(fadd(fmul(__ldg(m + 1), wd.x), fmul(__ldg(m + 5), wd.y)), fmul(__ldg(m + 9), wd.z)),
+                 fmul(__ldg(m + 13), 0.0f));
+    r.d.z = fadd(fadd(fadd(fmul(__ldg(m + 2), wd.x), fmul(__ldg(m + 6), wd.y)), fmul(__ldg(m + 10), wd.z)),
+                 fmul(__ldg(m + 14), 0.0f));
+    r.rd = recip3(r.d);
+}
+
 template <class STK, int TSTACK>
 struct SceneTrav {
     TravT<STK> bt;
@@ -784,20 +803,7 @@ struct SceneTrav {
                 return kStepFinished;
             }
             if (lr == 0u) {  // TLAS leaf: SceneObject::intersect
-                const float* m = sd.inv + 16ull * bl;
-                r.o.x = fadd(fadd(fadd(fmul(__ldg(m + 0), wo.x), fmul(__ldg(m + 4), wo.y)), fmul(__ldg(m + 8), wo.z)),
-                             fmul(__ldg(m + 12), 1.0f));
-                r.o.y = fadd(fadd(fadd(fmul(__ldg(m + 1), wo.x), fmul(__ldg(m + 5), wo.y)), fmul(__ldg(m + 9), wo.z)),
-                             fmul(__ldg(m + 13), 1.0f));
-                r.o.z = fadd(fadd(fadd(fmul(__ldg(m + 2), wo.x), fmul(__ldg(m + 6), wo.y)), fmul(__ldg(m + 10), wo.z)),
-                             fmul(__ldg(m + 14), 1.0f));
-                r.d.x = fadd(fadd(fadd(fmul(__ldg(m + 0), wd.x), fmul(__ldg(m + 4), wd.y)), fmul(__ldg(m + 8), wd.z)),
-                             fmul(__ldg(m + 12), 0.0f));
-                r.d.y = fadd(fadd(fadd(fmul(__ldg(m + 1), wd.x), fmul(__ldg(m + 5), wd.y)), fmul(__ldg(m + 9), wd.z)),
-                             fmul(__ldg(m + 13), 0.0f));
-                r.d.z = fadd(fadd(fadd(fmul(__ldg(m + 2), wd.x), fmul(__ldg(m + 6), wd.y)), fmul(__ldg(m + 10), wd.z)),
-                             fmul(__ldg(m + 14), 0.0f));
-                r.rd = recip3(r.d);
+                to_model(sd.inv + 16ull * bl, wo, wd, r);
                 r.inst_cur = bl;
                 blas = sd.blas_table[__ldg(sd.obj_blas + bl)];
                 bt.init(blas);
@@ -901,15 +907,46 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace_scene(SceneData sd, const
     if (active) store_hit(hits, i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, r.inst);
 }
 
-// PathTracer::evaluate over a whole scene (renderer.rs:345-384 -> Scene::intersect, scene.rs:32-34):
-// one 64-thread block per 8x8 tile, the camera ray through the pixel's top-left corner, the two-level
-// traversal of k_trace_scene, then the accumulator and shader.  The normal and texture accumulators
+// The accumulator and shader of a render over a scene.  The normal and texture accumulators
 // look up `scene.get_unchecked(instance_index)` (renderer.rs:258-263, 312-317): with lookup 0 the
 // reference's packed index -- instance 0, because Bvh::intersect packs instance 0
 // (InstancePrimitiveIndex::from_primitive, bvh.rs:296), and the primitive's low 20 bits
 // (intersection.rs:57-60) -- with lookup 1 the hit's own object.  A primitive outside the looked-up
 // model's data (where the reference's slice indexing panics) or missing shading data sets kErrLookup
 // and the pixel's radiance is zero.
+__device__ __forceinline__ void shade_scene_pixel(const SceneData& sd, const RenderParams& P,
+                                                  const ShadeEntry* __restrict__ shade_tab,
+                                                  const float* __restrict__ xf, int lookup, const LaneRay& r, int x, int y,
+                                                  uint8_t* __restrict__ rgba, uint32_t* err) {
+    const bool hit = r.hit && r.ct < FLT_MAX;
+    const float* nrm = nullptr;
+    const float* tc = nullptr;
+    const uint8_t* tex = nullptr;
+    uint32_t tw = 0, th = 0, prim = r.hp;
+    const float* oxf = xf;
+    bool ok = true;
+    if (hit && (P.acc_kind == BVHGPU_ACC_NORMAL || P.acc_kind == BVHGPU_ACC_TEXTURE)) {
+        const uint32_t obj = lookup ? r.inst : 0u;
+        prim = lookup ? r.hp : (r.hp & 0x000FFFFFu);
+        const ShadeEntry e = shade_tab[__ldg(sd.obj_blas + obj)];
+        oxf = xf + 16ull * obj;
+        nrm = e.normals;
+        tc = e.tex_coords;
+        tex = e.texels;
+        tw = e.tex_w;
+        th = e.tex_h;
+        ok = prim < e.ntris && (P.acc_kind == BVHGPU_ACC_NORMAL ? nrm != nullptr
+                                                                : (tc != nullptr && tex != nullptr && tw && th));
+        if (!ok) atomicOr(err, kErrLookup);
+    }
+    const float3 rad = ok ? accumulate(P, hit, r.ct, r.hu, r.hv, prim, nrm, oxf, tc, tex, tw, th)
+                          : make_float3(0.0f, 0.0f, 0.0f);
+    reinterpret_cast<uchar4*>(rgba)[(size_t)y * P.width + x] = shade(P, rad);
+}
+
+// PathTracer::evaluate over a whole scene (renderer.rs:345-384 -> Scene::intersect, scene.rs:32-34):
+// one 64-thread block per 8x8 tile, the camera ray through the pixel's top-left corner, the two-level
+// traversal of k_trace_scene, then the accumulator and shader.
 template <int STACK>
 __global__ void __launch_bounds__(64) k_render_scene(SceneData sd, RenderParams P,
                                                      const ShadeEntry* __restrict__ shade_tab,
@@ -945,30 +982,133 @@ __global__ void __launch_bounds__(64) k_render_scene(SceneData sd, RenderParams 
         scene_coop_phase(pend, tr, r, st);
     }
     if (!active) return;
-    const bool hit = r.hit && r.ct < FLT_MAX;
-    const float* nrm = nullptr;
-    const float* tc = nullptr;
-    const uint8_t* tex = nullptr;
-    uint32_t tw = 0, th = 0, prim = r.hp;
-    const float* oxf = xf;
-    bool ok = true;
-    if (hit && (P.acc_kind == BVHGPU_ACC_NORMAL || P.acc_kind == BVHGPU_ACC_TEXTURE)) {
-        const uint32_t obj = lookup ? r.inst : 0u;
-        prim = lookup ? r.hp : (r.hp & 0x000FFFFFu);
-        const ShadeEntry e = shade_tab[__ldg(sd.obj_blas + obj)];
-        oxf = xf + 16ull * obj;
-        nrm = e.normals;
-        tc = e.tex_coords;
-        tex = e.texels;
-        tw = e.tex_w;
-        th = e.tex_h;
-        ok = prim < e.ntris && (P.acc_kind == BVHGPU_ACC_NORMAL ? nrm != nullptr
-                                                                : (tc != nullptr && tex != nullptr && tw && th));
-        if (!ok) atomicOr(err, kErrLookup);
+    shade_scene_pixel(sd, P, shade_tab, xf, lookup, r, x, y, rgba, err);
+}
+
+// ---- one warp per ray (wide.cuh) over a scene ----------------------------------------------------
+struct WideSceneSmem {
+    WideSmem blas;
+    uint2 tlas[kWideTlas];
+};
+
+// The closest hit of world ray r (every lane the same) in the scene; r ends in the last visited object's
+// model space.  False: stopped, as wide_blas.
+__device__ __forceinline__ bool wide_scene(const SceneData& sd, LaneRay& r, LeafPolicy pol, WideSceneSmem& sm,
+                                           const Deadline& deadline, uint32_t* err) {
+    const unsigned lane = threadIdx.x & 31u;
+    const float3 wo = r.o, wd = r.d, wrd = r.rd;
+    uint32_t lr = __float_as_uint(__ldg(sd.tlas).w), bl = __float_as_uint(__ldg(sd.tlas + 1).w), tsteps = 0u, tsp = 0u;
+    for (;;) {
+        if (++tsteps > 2u * sd.tlas_nodes + 16u) {
+            if (lane == 0u) atomicOr(err, kErrSteps);
+            return false;
+        }
+        bool pop = true;
+        if (lr == 0u) {
+            to_model(sd.inv + 16ull * bl, wo, wd, r);
+            r.inst_cur = bl;
+            const GBlas b = sd.blas_table[__ldg(sd.obj_blas + bl)];
+            if (!wide_blas(b, r, pol, sm.blas, deadline, err)) return false;
+        } else {
+            const uint32_t li = (lr & 0xFFFF0000u) >> 16, ri = lr & 0xFFFFu;  // the swapped getters (tlas.rs:24-32)
+            const float4 l0 = __ldg(sd.tlas + 2ull * li), l1 = __ldg(sd.tlas + 2ull * li + 1);
+            const float4 r0 = __ldg(sd.tlas + 2ull * ri), r1 = __ldg(sd.tlas + 2ull * ri + 1);
+            float dl, dr;
+            const bool hl = slab(l0, l1, wo, wrd, r.ct, dl);
+            const bool hr = slab(r0, r1, wo, wrd, r.ct, dr);
+            const bool left_near = (hl ? dl : FLT_MAX) < (hr ? dr : FLT_MAX);
+            if (left_near ? hl : hr) {
+                if (left_near ? hr : hl) {
+                    if (tsp >= kWideTlas) {
+                        if (lane == 0u) atomicOr(err, kErrStack);
+                        return false;
+                    }
+                    if (lane == 0u)
+                        sm.tlas[tsp] = left_near ? make_uint2(ubits(r0.w), ubits(r1.w)) : make_uint2(ubits(l0.w), ubits(l1.w));
+                    ++tsp;
+                    __syncwarp();
+                }
+                lr = left_near ? ubits(l0.w) : ubits(r0.w);
+                bl = left_near ? ubits(l1.w) : ubits(r1.w);
+                pop = false;
+            }
+        }
+        if (pop) {
+            if (tsp == 0u) return true;
+            const uint2 e = sm.tlas[--tsp];
+            lr = e.x;
+            bl = e.y;
+            __syncwarp();
+        }
     }
-    const float3 rad = ok ? accumulate(P, hit, r.ct, r.hu, r.hv, prim, nrm, oxf, tc, tex, tw, th)
-                          : make_float3(0.0f, 0.0f, 0.0f);
-    reinterpret_cast<uchar4*>(rgba)[(size_t)y * P.width + x] = shade(P, rad);
+}
+
+__device__ __forceinline__ void init_scene_ray(LaneRay& r, float3 o, float3 d, float t) {
+    init_lane_ray(r, o, d, t);
+    r.inst = r.inst_cur = 0;
+}
+
+__global__ void __launch_bounds__(32 * kWideWarps) k_trace_scene_wide(SceneData sd, const float4* __restrict__ rays, uint32_t n,
+                                                                      GHit* __restrict__ hits, LeafPolicy pol, uint32_t* err) {
+    __shared__ WideSceneSmem smem[kWideWarps];
+    const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
+    if (i >= n) return;
+    LaneRay r;
+    float3 o, d;
+    float t0;
+    load_ray(rays, i, o, d, t0);
+    init_scene_ray(r, o, d, t0);
+    wide_scene(sd, r, pol, smem[threadIdx.x >> 5], Deadline{0ull}, err);
+    if ((threadIdx.x & 31u) == 0u) store_hit(hits, i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, r.inst);
+}
+
+__global__ void __launch_bounds__(32 * kWideWarps) k_render_scene_wide(SceneData sd, RenderParams P,
+                                                                       const ShadeEntry* __restrict__ shade_tab,
+                                                                       const float* __restrict__ xf, int lookup,
+                                                                       uint8_t* __restrict__ rgba, LeafPolicy pol, uint32_t* err) {
+    __shared__ WideSceneSmem smem[kWideWarps];
+    const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
+    if (i >= (uint32_t)P.width * (uint32_t)P.height) return;
+    const int x = (int)(i % (uint32_t)P.width), y = (int)(i / (uint32_t)P.width);
+    float3 o, d;
+    camera_ray(P, x, y, o, d);
+    LaneRay r;
+    init_scene_ray(r, o, d, FLT_MAX);
+    wide_scene(sd, r, pol, smem[threadIdx.x >> 5], Deadline{0ull}, err);
+    if ((threadIdx.x & 31u) == 0u) shade_scene_pixel(sd, P, shade_tab, xf, lookup, r, x, y, rgba, err);
+}
+
+__global__ void __launch_bounds__(32 * kWideWarps) k_scene_bounce_wide(SceneData sd, const float4* __restrict__ rays, uint32_t n,
+                                                                       uint32_t seed, GHit* __restrict__ hits0,
+                                                                       GHit* __restrict__ hits1, LeafPolicy pol, uint32_t* err) {
+    __shared__ WideSceneSmem smem[kWideWarps];
+    WideSceneSmem& sm = smem[threadIdx.x >> 5];
+    const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
+    const bool first = (threadIdx.x & 31u) == 0u;
+    if (i >= n) return;
+    Deadline deadline;
+    deadline.start(err);
+    LaneRay r;
+    float3 o, d;
+    float t0;
+    load_ray(rays, i, o, d, t0);
+    init_scene_ray(r, o, d, t0);
+    wide_scene(sd, r, pol, sm, deadline, err);
+    const bool h = r.hit && r.ct < FLT_MAX;
+    if (first) store_hit(hits0, i, h, r.ct, r.hu, r.hv, r.hp, r.inst);
+    float3 po, pd;
+    bool have = false;
+    if (h) {
+        const float4* T = sd.blas_table[__ldg(sd.obj_blas + r.inst)].tris + 3ull * r.hp;
+        have = bounce_dir_instanced(o, d, r.ct, __ldg(T + 1), __ldg(T + 2), sd.inv + 16ull * r.inst, seed, i, po, pd);
+    }
+    if (!have) {
+        if (first) store_hit(hits1, i, false, 0, 0, 0, 0, 0);
+        return;
+    }
+    init_scene_ray(r, po, pd, FLT_MAX);
+    wide_scene(sd, r, pol, sm, deadline, err);
+    if (first) store_hit(hits1, i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, r.inst);
 }
 
 // Persistent primary + bounce over a scene (the instanced frame): idle lanes are refilled from
@@ -1234,6 +1374,12 @@ cudaError_t launch_trace_scene(bvhgpu_ctx* ctx, DeviceScene& sc, const float4* r
     SceneData sd = scene_data(ctx, sc, &depth);
     LaunchScope scope(ctx, BVHGPU_K_TRACE_SCENE, s);
     const Variant v = resolve(ctx->tune[BVHGPU_K_TRACE_SCENE], depth);
+    if (n <= wide_rays(ctx, BVHGPU_K_TRACE_SCENE, sc.instanced_tris)) {
+        k_trace_scene_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(sd, rays, n, static_cast<GHit*>(hits), v.pol,
+                                                                               ctx->d_err);
+        g_launches++;
+        return cudaGetLastError();
+    }
     cudaError_t e = with_variant(v.shape, v.stack, [&](auto sh, auto tg) {
         using SH = decltype(sh);
         using STK = typename decltype(tg)::type;
@@ -1255,6 +1401,13 @@ cudaError_t launch_render_scene(bvhgpu_ctx* ctx, DeviceScene& sc, const bvhgpu_c
     const LeafPolicy pol = resolve(ctx->tune[BVHGPU_K_TRACE_SCENE], depth).pol;
     const unsigned tiles = (unsigned)(((w + 7) / 8) * ((h + 7) / 8));
     LaunchScope scope(ctx, BVHGPU_K_RENDER, s);
+    const uint64_t px = (uint64_t)w * (uint64_t)h;
+    if (px <= wide_rays(ctx, BVHGPU_K_TRACE_SCENE, sc.instanced_tris)) {
+        k_render_scene_wide<<<grid_for((uint32_t)px, kWideWarps), 32 * kWideWarps, 0, s>>>(sd, P, d_shade, sc.xf, lookup, d_rgba,
+                                                                                           pol, ctx->d_err);
+        g_launches++;
+        return cudaGetLastError();
+    }
     // the smallest local stack that holds the deepest BLAS's pending far children
     if (depth <= 33)
         k_render_scene<32><<<tiles, 64, 0, s>>>(sd, P, d_shade, sc.xf, lookup, d_rgba, pol, ctx->d_err);
@@ -1273,11 +1426,18 @@ cudaError_t launch_scene_bounce(bvhgpu_ctx* ctx, DeviceScene& sc, const float4* 
     if (n == 0) return cudaSuccess;
     uint32_t depth = 1;
     SceneData sd = scene_data(ctx, sc, &depth);
+    const Variant v = resolve(ctx->tune[BVHGPU_K_SCENE_BOUNCE], depth);
+    if (n <= wide_rays(ctx, BVHGPU_K_SCENE_BOUNCE, sc.instanced_tris)) {
+        LaunchScope scope(ctx, BVHGPU_K_SCENE_BOUNCE, s);
+        k_scene_bounce_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(sd, rays, n, seed, static_cast<GHit*>(hits0),
+                                                                                static_cast<GHit*>(hits1), v.pol, ctx->d_err);
+        g_launches++;
+        return cudaGetLastError();
+    }
     uint32_t* queue = ctx->d_scratch + 4;
     cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
     LaunchScope scope(ctx, BVHGPU_K_SCENE_BOUNCE, s);
-    const Variant v = resolve(ctx->tune[BVHGPU_K_SCENE_BOUNCE], depth);
     e = with_variant(v.shape, v.stack, [&](auto sh, auto tg) {
         using SH = decltype(sh);
         using STK = typename decltype(tg)::type;

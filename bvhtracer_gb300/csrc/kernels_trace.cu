@@ -17,6 +17,7 @@
 #include "persistent.cuh"
 #include "render.cuh"
 #include "variants.cuh"
+#include "wide.cuh"
 
 namespace bvhgpu {
 
@@ -100,130 +101,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace_blas(GBlas b, const float
     if (active) store_hit(hits, out_index ? out_index[i] : i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, 0u);
 }
 
-// ---- one warp per ray ----------------------------------------------------------------------
-// For launches of few rays (wide_rays): one thread per ray leaves most of the GPU idle and its time
-// is one lane's walk, so here a warp takes one ray.  Every lane follows the same reference nodes in
-// the reference's order; a leaf is tested by all lanes at once, small leaves (or leaves whose margins
-// are too wide) in order as in coop_leaf, large ones through their hidden tree: up to 8 nodes' children
-// are tested per iteration, one box per lane, and the live leaves' pairs one per lane.  Any order
-// of testing inside a leaf is exact (smallest t, ties to the lowest index; a hit from an earlier leaf
-// keeps equal t out).  What bounds it: the latency of the dependent node loads of one ray.
-constexpr uint32_t kWideStack = 256;    // pending reference nodes, as the largest stack variant
-constexpr uint32_t kWideNodes = 224;    // pending hidden nodes; fuller: the leaf is tested in order
-constexpr uint32_t kWideLeaves = 96;    // live hidden leaves waiting to be tested
-constexpr uint32_t kLeafPairs = kHiddenLeafTris / 2u;    // pairs of a hidden leaf, at most
-constexpr uint32_t kLeavesPerRound = 32u / kLeafPairs;  // hidden leaves tested at once, one pair per lane
-constexpr int kWideWarps = 2;           // warps (rays) per block
-// Leaves of at most this many triangles are tested in order (8 rounds of 64).  4,000 camera rays
-// against a 4,096-triangle soup / a 20,480-triangle sphere: 13 / 15 us at 256, 512 and 1,024, 19 / 15
-// at 32, 13 / 27 at 1,500.
-constexpr uint32_t kWideInOrder = 512;
-
-struct WideSmem {
-    uint2 stack[kWideStack];
-    uint2 nodes[kWideNodes];
-    uint2 leaves[kWideLeaves];
-};
-
-// The warp's best hit of the leaf in every lane (smallest t, ties to the lowest index).
-__device__ __forceinline__ void wide_reduce(Best& b) {
-    // accepted t are positive, so their bits order as the values do; a lane without a hit holds the
-    // incoming t with index ~0
-    const uint32_t t = __reduce_min_sync(kFull, b.k == kMiss ? 0x7F800000u : __float_as_uint(b.t));
-    if (t == 0x7F800000u) return;
-    b.k = __reduce_min_sync(kFull, (b.k != kMiss && __float_as_uint(b.t) == t) ? b.k : kMiss);
-    b.t = __uint_as_float(t);
-}
-
-// Tests the leaf [first, first + cnt) in index order, pairs dealt over the lanes.
-__device__ __forceinline__ void wide_in_order(const GBlas& g, uint32_t first, uint32_t cnt, const LaneRay& r, Best& b) {
-    const unsigned lane = threadIdx.x & 31u;
-    const f2 OX = f2_pack(r.o.x, r.o.x), OY = f2_pack(r.o.y, r.o.y), OZ = f2_pack(r.o.z, r.o.z);
-    const f2 DX = f2_pack(r.d.x, r.d.x), DY = f2_pack(r.d.y, r.d.y), DZ = f2_pack(r.d.z, r.d.z);
-    const f2 Z = f2_neg_zero();
-    const uint32_t end = first + cnt;
-    for (uint32_t p = (first >> 1) + lane; p < (end + 1u) >> 1; p += 32u) {
-        const uint32_t kA = 2u * p;
-        const PairData pd = load_pair(g.pairs + 5ull * p);
-        b.take(ray_terms(pd, origin_terms(pd, OX, OY, OZ, Z), DX, DY, DZ, Z, kA >= first, kA + 1u < end), kA);
-    }
-}
-
-// Walks the hidden tree `root` under margins lc.  False: the node list overflowed (test in order).
-__device__ __forceinline__ bool wide_hidden(const GBlas& g, uint2 root, LeafCull& lc, const LaneRay& r, Best& b,
-                                            WideSmem& sm) {
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned below = (1u << lane) - 1u;
-    const f2 OX = f2_pack(r.o.x, r.o.x), OY = f2_pack(r.o.y, r.o.y), OZ = f2_pack(r.o.z, r.o.z);
-    const f2 DX = f2_pack(r.d.x, r.d.x), DY = f2_pack(r.d.y, r.d.y), DZ = f2_pack(r.d.z, r.d.z);
-    const f2 Z = f2_neg_zero();
-    uint32_t nn = 1u, nl = 0u;
-    if (lane == 0u) sm.nodes[0] = make_uint2(root.y, root.x);  // (count, first)
-    __syncwarp();
-    while (nn | nl) {
-        if (nn && nl + 32u <= kWideLeaves) {
-            // the children of the newest up to 8 nodes, one box per lane
-            const uint32_t take = min(nn, 8u);
-            nn -= take;
-            const uint32_t slot = lane >> 2, c = lane & 3u;
-            bool live = false;
-            uint2 e = make_uint2(0u, 0u);
-            if (slot < take) {
-                const uint2 nd = sm.nodes[nn + slot];
-                if (c <= ((nd.x >> kWideShift) & 3u)) {
-                    const float4* N = g.nodes + 2ull * (nd.y + c);
-                    const float4 lo = __ldg(N), hi = __ldg(N + 1);
-                    float te;
-                    live = hidden_box(lo, hi, r.rd, lc, te);
-                    e = make_uint2(ubits(hi.w), ubits(lo.w));
-                }
-            }
-            const bool leaf = (e.x & kHiddenLeaf) != 0u;
-            const unsigned ml = __ballot_sync(kFull, live && leaf), mn = __ballot_sync(kFull, live && !leaf);
-            if (nn + (uint32_t)__popc(mn) > kWideNodes) return false;
-            __syncwarp();  // the entries taken above have been read
-            if (live && leaf) sm.leaves[nl + __popc(ml & below)] = e;
-            if (live && !leaf) sm.nodes[nn + __popc(mn & below)] = e;
-            nl += (uint32_t)__popc(ml);
-            nn += (uint32_t)__popc(mn);
-            __syncwarp();
-            if (nn && nl < kLeavesPerRound) continue;
-        }
-        // the newest live leaves, one pair per lane
-        const uint32_t take = min(nl, kLeavesPerRound);
-        if (take == 0u) continue;
-        nl -= take;
-        const uint32_t slot = lane / kLeafPairs, q = lane % kLeafPairs;
-        if (slot < take) {
-            const uint2 e = sm.leaves[nl + slot];
-            if (q < (e.x & ~kHiddenLeaf)) {
-                const uint32_t p = e.y + q;
-                uint2 idx;
-                const PairData pd = load_hidden_pair(g.pairs + 5ull * p, idx);
-                const PairHit h = ray_terms(pd, origin_terms(pd, OX, OY, OZ, Z), DX, DY, DZ, Z, idx.x != kMiss, idx.y != kMiss);
-                if (h.okA && (h.tA < b.t || (h.tA == b.t && b.k != kMiss && idx.x < b.k))) {
-                    b.t = h.tA;
-                    b.k = idx.x;
-                }
-                if (h.okB && (h.tB < b.t || (h.tB == b.t && b.k != kMiss && idx.y < b.k))) {
-                    b.t = h.tB;
-                    b.k = idx.y;
-                }
-            }
-        }
-        __syncwarp();
-        wide_reduce(b);
-        lc.thi = leaf_thi(lc, b.t);
-    }
-    return true;
-}
+// ---- one warp per ray (wide.cuh) -------------------------------------------------------------
 
 __global__ void __launch_bounds__(32 * kWideWarps) k_trace_wide(GBlas g, const float4* __restrict__ rays, uint32_t n,
                                                                 GHit* __restrict__ hits, LeafPolicy pol,
                                                                 uint32_t* err) {
     __shared__ WideSmem smem[kWideWarps];
-    WideSmem& sm = smem[threadIdx.x >> 5];
-    const unsigned lane = threadIdx.x & 31u;
     const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
     if (i >= n) return;
     LaneRay r;
@@ -231,74 +114,46 @@ __global__ void __launch_bounds__(32 * kWideWarps) k_trace_wide(GBlas g, const f
     float t0;
     load_ray(rays, i, o, d, t0);
     init_lane_ray(r, o, d, t0);
-    uint32_t cnt = g.root_count, first = g.root_first, sp = 0u, steps = 0u;
-    const uint32_t max_steps = 2u * (g.nodes_used + g.ntris) + 16u;
-    for (;;) {
-        if (++steps > max_steps) {
-            if (lane == 0u) atomicOr(err, kErrSteps);
-            break;
-        }
-        bool pop = true;
-        if (cnt == 0u) {
-            const float4* N = g.nodes + 2ull * first;
-            const float4 l0 = __ldg(N), l1 = __ldg(N + 1), r0 = __ldg(N + 2), r1 = __ldg(N + 3);
-            float dl, dr;
-            const bool hl = slab(l0, l1, r.o, r.rd, r.ct, dl), hr = slab(r0, r1, r.o, r.rd, r.ct, dr);
-            const bool left_near = (hl ? dl : FLT_MAX) < (hr ? dr : FLT_MAX);
-            if (left_near ? hl : hr) {
-                if (left_near ? hr : hl) {
-                    if (sp >= kWideStack) {
-                        if (lane == 0u) atomicOr(err, kErrStack);
-                        break;
-                    }
-                    if (lane == 0u)
-                        sm.stack[sp] = left_near ? make_uint2(ubits(r1.w), ubits(r0.w)) : make_uint2(ubits(l1.w), ubits(l0.w));
-                    ++sp;
-                    __syncwarp();
-                }
-                cnt = left_near ? ubits(l1.w) : ubits(r1.w);
-                first = left_near ? ubits(l0.w) : ubits(r0.w);
-                pop = false;
-            }
-        } else {
-            Best b{r.ct, kMiss};
-            bool done = false;
-            if (cnt > kWideInOrder && g.hx != nullptr && pol.max_duv > 0.0f) {
-                const uint2 e = __ldg(g.hx + first);
-                if (e.x != 0u) {
-                    const float4 a = __ldg(g.cones + 2ull * (e.y & kConeMask)), q = __ldg(g.cones + 2ull * (e.y & kConeMask) + 1);
-                    const LeafCone cone = {a.x, a.y, a.z, a.w, q.x, q.y};
-                    LeafCull lc = leaf_cull(cull_ray_rd(r.o.x, r.o.y, r.o.z, r.d.x, r.d.y, r.d.z, r.rd.x, r.rd.y, r.rd.z),
-                                            q.z, q.w, r.ct, pol.max_duv, cone);
-                    if (lc.on) {
-                        done = wide_hidden(g, e, lc, r, b, sm);
-                        if (!done) b = Best{r.ct, kMiss};
-                        __syncwarp();
-                    }
-                }
-            }
-            if (!done) wide_in_order(g, first, cnt, r, b);
-            wide_reduce(b);
-            if (b.k != kMiss) {
-                const float4* T = g.tris + 3ull * b.k;
-                float t, u, v;
-                tri_test(__ldg(T), __ldg(T + 1), __ldg(T + 2), r.o, r.d, t, u, v);  // the winner's u, v
-                r.ct = b.t;
-                r.hu = u;
-                r.hv = v;
-                r.hp = b.k;
-                r.hit = true;
-            }
-        }
-        if (pop) {
-            if (sp == 0u) break;
-            const uint2 e = sm.stack[--sp];
-            cnt = e.x;
-            first = e.y;
-            __syncwarp();
-        }
+    wide_blas(g, r, pol, smem[threadIdx.x >> 5], Deadline{0ull}, err);
+    if ((threadIdx.x & 31u) == 0u) store_hit(hits, i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, 0u);
+}
+
+// A primary and, where it hits, its diffuse bounce, by the same warp.
+__global__ void __launch_bounds__(32 * kWideWarps) k_bounce_wide(GBlas b, const float4* __restrict__ rays, uint32_t n,
+                                                                 uint32_t seed, GHit* __restrict__ hits0,
+                                                                 GHit* __restrict__ hits1, LeafPolicy pol, uint32_t key0,
+                                                                 uint32_t* hit_count, uint32_t* err) {
+    __shared__ WideSmem smem[kWideWarps];
+    WideSmem& sm = smem[threadIdx.x >> 5];
+    const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
+    const bool first = (threadIdx.x & 31u) == 0u;
+    if (i >= n) return;
+    Deadline dl;
+    dl.start(err);
+    LaneRay r;
+    float3 o, d;
+    float t0;
+    load_ray(rays, i, o, d, t0);
+    init_lane_ray(r, o, d, t0);
+    wide_blas(b, r, pol, sm, dl, err);
+    const bool h = r.hit && r.ct < FLT_MAX;
+    if (first) {
+        store_hit(hits0, i, h, r.ct, r.hu, r.hv, r.hp, 0u);
+        if (h && hit_count) atomicAdd(hit_count, 1u);
     }
-    if (lane == 0u) store_hit(hits, i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, 0u);
+    float3 po, pd;
+    bool have = false;
+    if (h) {
+        const float4* T = b.tris + 3ull * r.hp;
+        have = bounce_dir(r.o, r.d, r.ct, __ldg(T), __ldg(T + 1), __ldg(T + 2), seed, key0 + i, po, pd);
+    }
+    if (!have) {
+        if (first) store_hit(hits1, i, false, 0, 0, 0, 0, 0);
+        return;
+    }
+    init_lane_ray(r, po, pd, FLT_MAX);
+    wide_blas(b, r, pol, sm, dl, err);
+    if (first) store_hit(hits1, i, r.hit && r.ct < FLT_MAX, r.ct, r.hu, r.hv, r.hp, 0u);
 }
 
 // The plain traversal with per-ray work counters (one variant: block 128, local stack), summed
@@ -655,6 +510,23 @@ __global__ void __launch_bounds__(64) k_render(GBlas b, RenderParams P, const fl
     reinterpret_cast<uchar4*>(rgba)[(size_t)y * P.width + x] = shade(P, rad);
 }
 
+// The same for few pixels: one warp per pixel (wide.cuh).
+__global__ void __launch_bounds__(32 * kWideWarps) k_render_wide(GBlas b, RenderParams P, const float* __restrict__ normals,
+                                                                 uint8_t* __restrict__ rgba, LeafPolicy pol, uint32_t* err) {
+    __shared__ WideSmem smem[kWideWarps];
+    const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
+    if (i >= (uint32_t)P.width * (uint32_t)P.height) return;
+    float3 o, d;
+    camera_ray(P, (int)(i % (uint32_t)P.width), (int)(i / (uint32_t)P.width), o, d);
+    LaneRay lr;
+    init_lane_ray(lr, o, d, FLT_MAX);
+    wide_blas(b, lr, pol, smem[threadIdx.x >> 5], Deadline{0ull}, err);
+    if ((threadIdx.x & 31u) != 0u) return;
+    const float3 rad = accumulate(P, lr.hit && lr.ct < FLT_MAX, lr.ct, lr.hu, lr.hv, lr.hp, normals, P.acc, P.tex_coords,
+                                  P.texels, P.tex_w, P.tex_h);
+    reinterpret_cast<uchar4*>(rgba)[i] = shade(P, rad);
+}
+
 }  // namespace
 
 #define BVHGPU_DISPATCH_STACK(depth, ...)                         \
@@ -679,19 +551,6 @@ static cudaError_t trace_blas_variant(bvhgpu_ctx* ctx, const Variant& v, const G
     });
 }
 
-// Launches of at most this many rays run one warp per ray (under the default launch config only: a
-// config set by the caller or the tuner names the one-thread kernel's variants).  Measured against the
-// one-thread kernel, in us, at 8,000 / 16,000 / 32,000 / 64,000 camera rays (random rays gain more): soup of
-// 300 triangles 24 | 24 | 43 | 43 -> 23 | 37 | 85 | 143; sphere of 320 23 | 23 | 27 | 29 -> 16 | 25 |
-// 50 | 86; sphere of 5,120 58 | 72 | 72 | 74 -> 21 | 35 | 62 | 114; soup of 4,096 123 | 199 | 260 |
-// 293 -> 24 | 39 | 81 | 134; sphere of 81,920 194 | 203 | 203 | 248 -> 30 | 43 | 78 | 140.  The one-thread
-// kernel's time hardly grows until the GPU is full and then starts from the mesh's longest walk, so
-// the line lies higher for larger meshes.
-static uint32_t wide_rays(const bvhgpu_ctx* ctx, const DeviceBlas& b) {
-    if (!default_tune(ctx->tune[BVHGPU_K_TRACE_BLAS], BVHGPU_K_TRACE_BLAS)) return 0u;
-    return b.ntris < 4096u ? 8192u : 32768u;
-}
-
 cudaError_t launch_trace_blas(bvhgpu_ctx* ctx, const DeviceBlas& b, const float4* rays, uint32_t n, void* hits,
                               cudaStream_t s) {
     if (n == 0) return cudaSuccess;
@@ -699,7 +558,7 @@ cudaError_t launch_trace_blas(bvhgpu_ctx* ctx, const DeviceBlas& b, const float4
     LaunchScope scope(ctx, BVHGPU_K_TRACE_BLAS, s);
     const Variant v = resolve(ctx->tune[BVHGPU_K_TRACE_BLAS], b.depth);
     cudaError_t e;
-    if (n <= wide_rays(ctx, b)) {
+    if (n <= wide_rays(ctx, BVHGPU_K_TRACE_BLAS, b.ntris, 8192u)) {
         k_trace_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(g, rays, n, static_cast<GHit*>(hits), v.pol,
                                                                          ctx->d_err);
         e = cudaGetLastError();
@@ -742,12 +601,19 @@ cudaError_t launch_bounce_persistent(bvhgpu_ctx* ctx, const DeviceBlas& b, const
                                      uint32_t seed, void* hits0, void* hits1, cudaStream_t s, uint32_t base,
                                      uint32_t* hit_count) {
     if (n == 0) return cudaSuccess;
+    GBlas g = to_gblas(b);
+    const Variant v = resolve(ctx->tune[BVHGPU_K_PERSISTENT_BOUNCE], b.depth);
+    if (n <= wide_rays(ctx, BVHGPU_K_PERSISTENT_BOUNCE, b.ntris)) {
+        LaunchScope scope(ctx, BVHGPU_K_PERSISTENT_BOUNCE, s);
+        k_bounce_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(
+            g, rays, n, seed, static_cast<GHit*>(hits0), static_cast<GHit*>(hits1), v.pol, base, hit_count, ctx->d_err);
+        g_launches++;
+        return cudaGetLastError();
+    }
     uint32_t* queue = ctx->d_scratch + 2;
     cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    GBlas g = to_gblas(b);
     LaunchScope scope(ctx, BVHGPU_K_PERSISTENT_BOUNCE, s);
-    const Variant v = resolve(ctx->tune[BVHGPU_K_PERSISTENT_BOUNCE], b.depth);
     e = with_variant(v.shape, v.stack, [&](auto sh, auto tg) {
         using SH = decltype(sh);
         using STK = typename decltype(tg)::type;
@@ -890,6 +756,13 @@ cudaError_t launch_render(bvhgpu_ctx* ctx, const DeviceBlas& b, const bvhgpu_cam
     GBlas g = to_gblas(b);
     unsigned tiles = (unsigned)(((w + 7) / 8) * ((h + 7) / 8));
     LaunchScope scope(ctx, BVHGPU_K_RENDER, s);
+    const uint64_t px = (uint64_t)w * (uint64_t)h;
+    if (px <= wide_rays(ctx, BVHGPU_K_TRACE_BLAS, b.ntris)) {
+        k_render_wide<<<grid_for((uint32_t)px, kWideWarps), 32 * kWideWarps, 0, s>>>(
+            g, P, d_normals, d_rgba, resolve(ctx->tune[BVHGPU_K_TRACE_BLAS], b.depth).pol, ctx->d_err);
+        g_launches++;
+        return cudaGetLastError();
+    }
     BVHGPU_DISPATCH_STACK(b.depth, (k_render<S><<<tiles, 64, 0, s>>>(g, P, d_normals, d_rgba, resolve(ctx->tune[BVHGPU_K_TRACE_BLAS], b.depth).pol, ctx->d_err)));
     g_launches++;
     return cudaGetLastError();

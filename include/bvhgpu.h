@@ -422,7 +422,8 @@ int bvhgpu_mesh_update_async(bvhgpu_ctx* ctx, uint32_t mesh_id, bvhgpu_stream s)
 /* Forward: closest hit per ray, hit records {t, u, v, prim} written to d_hits (the checkpoint the
  * adjoint reuses), image[i] = max(0, n_hat . l_hat) with n the barycentric vertex normal and l the
  * direction from the hit point to the point light `light` (0 for a miss).  One persistent launch
- * under the BVHGPU_K_TRACE_BLAS launch config (shape, stack, leaf policy, refill).  Each pass
+ * under the BVHGPU_K_TRACE_BLAS launch config (shape, stack, leaf policy, refill), or one warp per
+ * ray for few rays.  Each persistent pass
  * records which rays took long to trace, and the mesh's next pass starts those first, spread over
  * the launch (results never depend on it); the record takes 16 bytes per ray, allocated by the first
  * pass at a larger ray count (outside stream capture; a captured pass that finds it too small runs
@@ -469,9 +470,10 @@ typedef struct bvhgpu_tune_config {
     uint32_t hidden;
 } bvhgpu_tune_config;
 /* Defaults (the tuner's picks on GB300): block 128, min_blocks 5, stack 256, big_leaf 16, refill 8,
- * hidden 2000; for the single-ray kernels (TRACE_BLAS, TRACE_SCENE) refill 1.  While TRACE_BLAS has its
- * default config (hidden may be any value from 1000 on), launches of few rays run one warp per ray
- * instead (same hits). */
+ * hidden 2000; for the single-ray kernels (TRACE_BLAS, TRACE_SCENE) refill 1.  While a kernel has its
+ * default config (hidden may be any value from 1000 on), its launches of few rays run one warp per ray
+ * instead (same results; renders and the Lambertian forward pass follow TRACE_BLAS, scene renders
+ * TRACE_SCENE). */
 int bvhgpu_tune_get(bvhgpu_ctx* ctx, int kernel, bvhgpu_tune_config* out);
 /* BVHGPU_ERR_INVALID_ARG for a kernel that is not tunable or a shape / stack not compiled. */
 int bvhgpu_tune_set(bvhgpu_ctx* ctx, int kernel, const bvhgpu_tune_config* cfg);
