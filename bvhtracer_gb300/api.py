@@ -123,7 +123,7 @@ class Context:
     def trace_batch(self, items, rays: np.ndarray, mode: int) -> np.ndarray:
         items = np.ascontiguousarray(items, BATCH_ITEM)
         rays = np.ascontiguousarray(rays, RAY)
-        hits = np.zeros(len(rays), HIT)
+        hits = np.empty(len(rays), HIT)
         self.check(self.lib.bvhgpu_trace_batch(self.h, ptr(items), len(items), ptr(rays), len(rays), mode,
                                                ptr(hits)))
         return hits
@@ -157,7 +157,7 @@ class Context:
         against a triangle list in index order, no BVH."""
         tris = np.ascontiguousarray(tris, np.float32).reshape(-1, 9)
         rays = np.ascontiguousarray(rays, RAY)
-        hits = np.zeros(len(rays), HIT)
+        hits = np.empty(len(rays), HIT)
         self.check(self.lib.bvhgpu_triangles_intersect(self.h, ptr(tris), len(tris), ptr(rays), len(rays), mode,
                                                        ptr(hits)))
         return hits
@@ -432,7 +432,7 @@ class Blas:
     def intersect(self, rays: np.ndarray) -> np.ndarray:
         """Bvh::intersect for every ray (host arrays in, host hits out)."""
         rays = np.ascontiguousarray(rays, RAY)
-        hits = np.zeros(len(rays), HIT)
+        hits = np.empty(len(rays), HIT)
         self.ctx.check(self.ctx.lib.bvhgpu_blas_intersect(self.ctx.h, self.id, ptr(rays), len(rays), ptr(hits)))
         return hits
 
@@ -442,8 +442,8 @@ class Blas:
 
     def trace_bounce(self, rays: np.ndarray, seed: int, mode: int):
         rays = np.ascontiguousarray(rays, RAY)
-        h0 = np.zeros(len(rays), HIT)
-        h1 = np.zeros(len(rays), HIT)
+        h0 = np.empty(len(rays), HIT)
+        h1 = np.empty(len(rays), HIT)
         nb = ctypes.c_uint32()
         self.ctx.check(self.ctx.lib.bvhgpu_blas_trace_bounce(self.ctx.h, self.id, ptr(rays), len(rays), seed, mode,
                                                              ptr(h0), ptr(h1), ctypes.byref(nb)))
@@ -599,7 +599,7 @@ class Scene:
 
     def intersect(self, rays: np.ndarray) -> np.ndarray:
         rays = np.ascontiguousarray(rays, RAY)
-        hits = np.zeros(len(rays), HIT)
+        hits = np.empty(len(rays), HIT)
         self.ctx.check(self.ctx.lib.bvhgpu_scene_intersect(self.ctx.h, self.id, ptr(rays), len(rays), ptr(hits)))
         return hits
 
