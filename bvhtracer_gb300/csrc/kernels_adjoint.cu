@@ -28,13 +28,12 @@ namespace {
 
 constexpr int kBlock = 128;
 constexpr unsigned kFull = 0xFFFFFFFFu;
-// The forward pass's long-ray schedule: a ray with more traversal steps than kLongSteps is served
-// first by the next pass, spread evenly over the launch's warps.  Measured on the 512 x 512
-// level-7 icosphere (median 21 steps, 99th percentile 395): 1.89 ms unscheduled; 1.64 ms at 250
-// steps; 1.66 / 1.72 / 1.72 ms at 300 / 200 / 400; fixed caps of 1-4 long rays per warp instead of
-// the even share 1.66-2.40 ms (long rays waiting for a free slot start late).
-constexpr uint32_t kLongSteps = 250;
-
+// The forward pass's long-ray schedule: a ray with more traversal steps than this is served first by the
+// next pass, spread evenly over the launch's warps.  Forward pass of 512 x 512 rays, four views of a
+// level-7 sphere, in us at 56 / 64 / 80 / 250 steps (250: where it stood with wider margins and longer
+// walks): 281 / 285 / 299 / 350 on average; 400 x 400, level 6: 198 / 207 / 221 / 238; 512 x 512, level 5: 210 / 205 /
+// 201 / 201 -- in small meshes most silhouette rays pass 64 steps, and a list of them all spreads nothing.
+__device__ __forceinline__ uint32_t long_steps(uint32_t ntris) { return ntris < 65536u ? 80u : 60u; }
 inline unsigned grid_for(uint32_t n, int block) { return (unsigned)((n + block - 1) / block); }
 
 inline GBlas to_gblas(const DeviceBlas& b) {
@@ -118,7 +117,7 @@ __global__ void k_mesh_tris(const float* __restrict__ verts, const uint32_t* __r
 // mesh or finished early take new pixels instead of idling until the slowest ray of their block
 // is done.  A finished pixel stores its hit record (the adjoint's checkpoint) and its intensity.
 //
-// Long rays (more than kLongSteps traversal steps: the silhouette's grazing rays, up to ~30x the
+// Long rays (more than long_steps traversal steps: the silhouette's grazing rays, up to ~30x the
 // median) sit side by side in pixel order, so a warp that draws a silhouette tile runs ~20 of them
 // divergently together and the launch's tail is that warp.  With a schedule (`sched`, ForwardSchedule
 // layout) each pass records its long rays, and the next pass serves them first from that list,
@@ -236,7 +235,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_lambert_forward(GBlas b, const 
                 }
                 image[idx] = I;
                 if (sched != nullptr) {
-                    const bool lng = tr.steps > kLongSteps;
+                    const bool lng = tr.steps > long_steps(b.ntris);
                     __stcg(flag_nxt + idx, lng ? 1u : 0u);
                     if (lng) {
                         const uint32_t slot = atomicAdd(ctr + ForwardSchedule::kCount + (parity ^ 1u), 1u);
