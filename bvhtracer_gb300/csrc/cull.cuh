@@ -57,7 +57,7 @@
 // rays with a non-finite or huge component or a tiny non-zero d_i (|1 / d_i| >= 1e20), and leaves
 // without a positive Dlo are never culled.  Audited on the CPU against the float test on
 // adversarial rays (aimed at edges and vertices, grazing the plane, axis-aligned): no culled box
-// held an accepted hit at or below t_best, and the largest measured error was 0.19 of its margin.
+// held an accepted hit at or below t_best, and the largest measured error was 0.21 of its margin (11.9 M hits).
 //
 // Counting the roundings term by term, instead of bounding each triple product by its largest
 // factors with a further factor 4 on every term, made R 50 to 100 times narrower.  With it hidden
