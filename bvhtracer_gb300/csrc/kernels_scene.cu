@@ -1324,7 +1324,9 @@ size_t tlas_work_bytes(uint32_t nobj) { return 7ull * sizeof(float) * nobj; }
 template <int B, int K>
 static cudaError_t tlas_rebuild_block(bvhgpu_ctx* ctx, DeviceScene& sc, cudaStream_t s) {
     const size_t smem = 32ull * sc.nobjects;
-    if (smem > 48u * 1024u) {
+    // the default limit covers the kernel's static shared memory (s_best) too
+    constexpr size_t kStatic = 2 * sizeof(unsigned long long) * (B / 32);
+    if (smem + kStatic > 48u * 1024u) {
         const cudaError_t e = cudaFuncSetAttribute(k_tlas_rebuild<B, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * B * K);
         if (e != cudaSuccess) return e;
     }

@@ -1,6 +1,10 @@
 """The TLAS rebuild's block variants (list in registers, 2 to 8 clusters a thread) against Tlas::rebuild
 bit for bit, at the edges of every variant's range, with exact area ties, with empty boxes, and where the
 reference would panic (no candidate below FLT_MAX)."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -69,3 +73,20 @@ def test_nobody_left_to_merge_with(model):
     xf, inv = placed(5, 9, False)
     xf[:, 12] = np.array([-3e38, 3e38, -1e38, 2e38, 0], np.float32)
     assert check(model, xf, inv) is None
+
+
+@pytest.mark.parametrize("n", [1532, 1533, 1536, 1537])
+def test_sizes_at_the_default_shared_memory_limit(n):
+    """1,533 objects fill 48 KB together with the block's own minima.  In a process of its own: a larger
+    scene raises the kernel's limit for the rest of its process."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = ("import bvhtracer_gb300 as bt\n"
+            "from bvhtracer_gb300 import scenes\n"
+            "from test_gpu_tlas_blocks import check, placed\n"
+            "tris = scenes.displaced_icosphere(1, 5).triangles().copy()\n"
+            "bvh = bt.BvhBuilder().build_for(tris)\n"
+            "ctx = bt.Context(0)\n"
+            f"assert check((ctx, ctx.upload_blas(bvh, tris), bvh.nodes[0]), *placed({n}, 3, False)) is not None\n")
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(here), here]))
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
