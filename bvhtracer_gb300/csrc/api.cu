@@ -111,7 +111,10 @@ volatile uint32_t* host_flags(bvhgpu_ctx* ctx) { return static_cast<uint32_t*>(c
 int read_errors(bvhgpu_ctx* ctx) {
     const uint32_t flags = *host_flags(ctx);
     if (flags) {
-        CK(cudaMemset(ctx->d_err, 0, sizeof(uint32_t)), "reset error flags");
+        // on the stream of the reads and launches, and done before the error is returned: a reset that is
+        // still pending would let the next call read this error again, or wipe one of its own
+        CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream), "reset error flags");
+        CK(cudaStreamSynchronize(ctx->stream), "reset error flags");
         if (flags & kErrStack) return fail(ctx, BVHGPU_ERR_STACK_DEPTH, "traversal stack overflow (tree too deep)");
         if (flags & kErrDeadline)
             return fail(ctx, BVHGPU_ERR_DEADLINE, "a launch stopped at the context's deadline; its outputs are incomplete");
