@@ -504,7 +504,7 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
         (e = cudaMalloc(&b.leaf_keys, 48ull * std::max<size_t>(1, leaves.size()))) != cudaSuccess ||
         (hx_bytes && (e = cudaMalloc(&b.hx, hx_bytes)) != cudaSuccess) ||
         (b.ncones && (e = cudaMalloc(&b.cones, 32ull * b.ncones)) != cudaSuccess) ||
-        (b.nhid && (e = cudaMalloc(&b.hup, 16ull * b.nhid)) != cudaSuccess) ||
+        (b.nhid && (e = cudaMalloc(&b.hup, 16ull * (b.nhid + b.nleaves))) != cudaSuccess) ||
         (b.nhid && (e = cudaMalloc(&b.hagg, 128ull * b.nhid)) != cudaSuccess) ||
         (b.nhid && (e = cudaMalloc(&b.harrivals, 4ull * b.nhid)) != cudaSuccess)) {
         cleanup();
@@ -521,8 +521,15 @@ int bvhgpu_blas_upload(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t nodes
         (e = cudaMemsetAsync(b.pairs, 0, 80ull * pairs_all, st)) != cudaSuccess ||
         (b.nhid && (e = cudaMemsetAsync(b.harrivals, 0, 4ull * b.nhid, st)) != cudaSuccess) ||
         (e = finish_hidden(ctx, hp, b, st)) != cudaSuccess ||
-        (e = launch_write_tris(ctx, b, static_cast<const float*>(d_tris9), st)) != cudaSuccess ||
+        (e = launch_write_tris(ctx, b, static_cast<const float*>(d_tris9), st, hp.decide)) != cudaSuccess ||
+        (b.nhid && (e = cudaMemcpyAsync(ctx->host_word, hp.decide, sizeof(uint32_t), cudaMemcpyDeviceToHost, st)) != cudaSuccess) ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess) {
+        cleanup();
+        return cuda_fail(ctx, e, "blas_upload");
+    }
+    b.measured_roots = b.nhid && *static_cast<const volatile uint32_t*>(ctx->host_word) != 0u;
+    if (b.measured_roots && ((e = launch_hidden_refresh(ctx, b, st, false, nullptr)) != cudaSuccess ||
+                             (e = cudaStreamSynchronize(st)) != cudaSuccess)) {
         cleanup();
         return cuda_fail(ctx, e, "blas_upload");
     }

@@ -32,11 +32,12 @@ struct DeviceBlas {
     uint2* hx = nullptr;         // hidden-tree table and pair slots (GBlas::hx), or null
     float4* cones = nullptr;     // hidden-tree cone records (GBlas::cones)
     uint32_t ncones = 0;
-    uint4* hup = nullptr;        // refresh links of each hidden node (k_hidden_refresh)
+    uint4* hup = nullptr;        // refresh links of each hidden node, then of each leaf (kernels_scene.cu)
     float4* hagg = nullptr;      // 8 float4 per hidden node: the refresh's aggregates
     uint32_t* harrivals = nullptr;  // per hidden node: the refresh's arrival counters (kept zeroed)
     uint32_t nhid = 0;           // hidden nodes (after the nodes_used reference nodes)
     uint32_t nhp = 0;            // hidden pairs (after the (ntris + 1) / 2 pairs in triangle order)
+    bool measured_roots = false; // the hidden roots' cones are measured over their triangles (set at upload)
     uint32_t ref_depth = 0;      // depth of the reference tree (depth adds the hidden trees')
     uint32_t nodes_used = 0;
     uint32_t ntris = 0;
@@ -57,6 +58,7 @@ struct HiddenPlan {
     void* work = nullptr;
     uint32_t nhid = 0, nhp = 0, ncones = 0, depth = 0, table_u2 = 0;
     uint32_t *ids = nullptr, *pair_at = nullptr, *sums = nullptr;
+    uint32_t* decide = nullptr;  // a zero word for the first refresh
     uint2 *meta = nullptr, *range = nullptr, *table = nullptr;
     uint4* up = nullptr;
 };
@@ -251,10 +253,12 @@ cudaError_t plan_hidden(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t node
 cudaError_t finish_hidden(bvhgpu_ctx* ctx, const HiddenPlan& plan, DeviceBlas& b, cudaStream_t s);
 
 // ---- launchers (kernels_scene.cu) ------------------------------------------------------
-cudaError_t launch_write_tris(bvhgpu_ctx* ctx, DeviceBlas& b, const float* d_tris9, cudaStream_t s);
+cudaError_t launch_write_tris(bvhgpu_ctx* ctx, DeviceBlas& b, const float* d_tris9, cudaStream_t s, uint32_t* decide = nullptr);
 // Rewrites the hidden trees' pairs, boxes and leaf bounds from b.tris; part of every triangle write.
-cudaError_t launch_hidden_refresh(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s);
-cudaError_t launch_refit(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s);
+// decide (device, may be null): set to 1 where the model's hidden roots need measured cones.  refit_follows: a
+// launch_refit with after_refresh follows on the stream and measures them in its own pass over the triangles.
+cudaError_t launch_hidden_refresh(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s, bool refit_follows, uint32_t* decide);
+cudaError_t launch_refit(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s, bool after_refresh = false);
 // Physics (physics.cu).
 cudaError_t launch_world_start_frame(bvhgpu_ctx* ctx, DeviceWorld& w, cudaStream_t s);
 cudaError_t launch_world_step(bvhgpu_ctx* ctx, DeviceWorld& w, float dt, cudaStream_t s);

@@ -372,8 +372,8 @@ cudaError_t launch_mesh_update(bvhgpu_ctx* ctx, DeviceMesh& m, DeviceBlas& b, cu
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if ((e = launch_hidden_refresh(ctx, b, s)) != cudaSuccess) return e;
-    return launch_refit(ctx, b, s);
+    if ((e = launch_hidden_refresh(ctx, b, s, true, nullptr)) != cudaSuccess) return e;
+    return launch_refit(ctx, b, s, true);
 }
 
 cudaError_t launch_lambert_forward(bvhgpu_ctx* ctx, DeviceMesh& m, const DeviceBlas& b, const float4* rays, uint32_t n,

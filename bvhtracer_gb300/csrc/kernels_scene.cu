@@ -59,7 +59,10 @@ __global__ void k_write_tris(const float* __restrict__ tris9, uint32_t n, float4
 //  - Boxes, Q and B are minima and maxima of the triangles' own values: the same in any order.
 //  - A node's normal cone is built from its grandchildren's cones: the axis is the sum of the children's
 //    folded unit-normal sums (any axis is valid), and normals within phi_c of the line of a grandchild's
-//    axis are within theta_c + phi_c of the line of the node's axis (theta_c between the axes).
+//    axis are within theta_c + phi_c of the line of the node's axis (theta_c between the axes).  That loosens
+//    with every level (roots over 3,400 triangles: 47 degrees where the normals span 40).  In models so large
+//    that a root's cone decides whether its leaf can be walked at all (cones_decide), the roots' cones are
+//    measured over their triangles instead (fold_root_cones).
 // The quad of lanes climbs together, a child per lane.  What bounds it: the climb's dependent hops (a
 // counter, a fence and up to four 128-B records each).
 // Against two passes of every node over all its triangles (a warp per 256 pairs), which read each
@@ -147,12 +150,22 @@ __device__ __forceinline__ float wider_cone(const float* a, const float* s, floa
     return c > 0.0f ? c : -1.0f;
 }
 
+// Whether the plain margin (leaf_cull) of a tree with bounds Q, B is too wide to walk it (2, the default limit)
+// already for rays from within 7 B of the origin: its cone alone then decides.  Below, the looser roots cost
+// nothing measurable, and the second pass over the triangles would (update of 20,480 triangles 25 -> 32 us).
+__device__ __forceinline__ bool cones_decide(float Q, float B) {
+    const float w = 2.0f * 1.7320508f * 8.0f * B;  // W of a unit direction along the diagonal
+    return !(8.0f * kCullUnit * w * Q + 28.0f * kCullUnit * 1.7320508f * 0.25f * Q * Q < 2.0f * 0.0001f);
+}
+
 // up[i] of hidden node i (both counted from the first hidden node): {first node of its sibling block,
-// siblings, parent node (kNoRefresh: a hidden root), the parent's cone record}.
+// siblings, parent node (kNoRefresh: a hidden root), the parent's cone record}.  measured: fold_root_cones
+// follows and makes the roots' cones.  decide (may be null): set to 1 where cones_decide.
 __global__ void __launch_bounds__(256) k_hidden_refresh(const float4* __restrict__ tris, const uint2* __restrict__ slots,
                                                         uint32_t p0, float4* __restrict__ pairs,
                                                         float4* nodes, uint32_t nhid, const uint4* __restrict__ up,
-                                                        float4* agg, uint32_t* arrivals, float4* __restrict__ cones) {
+                                                        float4* agg, uint32_t* arrivals, float4* __restrict__ cones, bool measured,
+                                                        uint32_t* decide) {
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, q = threadIdx.x & 3u;
     uint32_t first = 0u, count = 0u;
     if (i < nhid) {
@@ -233,7 +246,7 @@ __global__ void __launch_bounds__(256) k_hidden_refresh(const float4* __restrict
         __stcg(a + q, q == 0u   ? make_float4(g.lo[0], g.lo[1], g.lo[2], g.e1m)
                       : q == 1u ? make_float4(g.hi[0], g.hi[1], g.hi[2], g.e2m)
                       : q == 2u ? make_float4(g.s[0], g.s[1], g.s[2], g.cphi)
-                                : make_float4(g.nmin, g.finite, 0.0f, 0.0f));
+                                : make_float4(g.nmin, g.finite, kNoEntry, 0.0f));
         __stcg(a + 4u + q, entry);
         const uint4 u = up[cur];
         __threadfence();
@@ -265,6 +278,14 @@ __global__ void __launch_bounds__(256) k_hidden_refresh(const float4* __restrict
         }
         g.cphi = quad_min(cphi, quad);
         const GroupSeal seal = group_seal(g.lo, g.hi, g.e1m, g.e2m, g.finite != 0.0f);
+        if (u.z == kNoRefresh) {
+            if (decide != nullptr && q == 0u && cones_decide(seal.q, seal.b)) *decide = 1u;
+            if (measured) {  // the axis and the bounds
+                if (q == 0u) cones[2ull * u.w] = make_float4(g.s[0], g.s[1], g.s[2], -1.0f);
+                if (q == 1u) cones[2ull * u.w + 1] = make_float4(1.0f, g.nmin, seal.q, seal.b);
+                return;
+            }
+        }
         const bool ok = isfinite(g.s[0]) && isfinite(g.s[1]) && isfinite(g.s[2]) && g.cphi > 0.0f && g.cphi <= 1.0f &&
                         g.nmin > 0.0f && g.nmin < FLT_MAX;
         if (!ok) g.cphi = -1.0f;
@@ -273,6 +294,62 @@ __global__ void __launch_bounds__(256) k_hidden_refresh(const float4* __restrict
         if (u.z == kNoRefresh) return;
         cur = u.z;
     }
+}
+
+// The hidden roots' normal cones, measured: the least |cos| between any of a root's triangles' normals and its axis.
+// links[li] of reference leaf li: {first node of the root's children's block (kNone: no hidden tree), cone
+// record, triangles}.  Every lane brings one triangle (link: its leaf's; a leaf's triangles are consecutive,
+// so a warp's are mostly of one root); the warp folds them into the root's word, which the refresh left at
+// kNoEntry, and the last triangles to arrive finish the record.  Primaries of 400 x 400 from 3 radii, roots from
+// their grandchildren's cones | measured: 81,920-triangle sphere of radius 100 1,651 | 1,270 us, 20,480
+// triangles 465 | 360 us.
+__device__ __forceinline__ void fold_root_cones(uint4 link, const float* e1, const float* e2, float4* agg, uint32_t* arrivals,
+                                                float4* cones) {
+    const unsigned lane = threadIdx.x & 31u;
+    int cosine = 0x7FFFFFFF;  // a float's bits: they order as signed integers, and -1 is below all
+    if (link.x != kNone) {
+        const float4 a = __ldcg(cones + 2ull * link.y);
+        float cl, nl;
+        cone_terms(e1, e2, a.x, a.y, a.z, cl, nl);
+        cosine = __float_as_int(cl == cl ? cl : -1.0f);
+    }
+    unsigned todo = __ballot_sync(kFull, link.x != kNone);
+    while (todo) {
+        const int leader = __ffs(todo) - 1;
+        const uint32_t root = __shfl_sync(kFull, link.x, leader);
+        const unsigned group = __ballot_sync(kFull, link.x == root);
+        const int least = __reduce_min_sync(kFull, link.x == root ? cosine : 0x7FFFFFFF);
+        todo &= ~group;
+        if ((int)lane != leader) continue;
+        int* word = reinterpret_cast<int*>(agg + 8ull * root + 3u) + 2;
+        atomicMin(word, least);
+        __threadfence();
+        if (atomicAdd(arrivals + root, (uint32_t)__popc(group)) + (uint32_t)__popc(group) != link.z) continue;
+        __threadfence();
+        arrivals[root] = 0u;  // ready for the next refresh
+        const float c = __int_as_float(__ldcg(word));
+        const float4 a = __ldcg(cones + 2ull * link.y), b = __ldcg(cones + 2ull * link.y + 1);
+        const bool ok = isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && c > 0.0f && c <= 1.0f && b.y > 0.0f && b.y < FLT_MAX;
+        cones[2ull * link.y] = ok ? make_float4(a.x, a.y, a.z, c) : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+        cones[2ull * link.y + 1] = make_float4(ok ? cone_sin(c) : 1.0f, ok ? b.y : 0.0f, b.z, b.w);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_hidden_root_cones(const float4* __restrict__ tris, uint32_t ntris,
+                                                           const uint32_t* __restrict__ tri_leaf,
+                                                           const uint4* __restrict__ links, float4* agg, uint32_t* arrivals,
+                                                           float4* cones) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint4 link = make_uint4(kNone, 0u, 0u, 0u);
+    float e1[3] = {0.0f, 0.0f, 0.0f}, e2[3] = {0.0f, 0.0f, 0.0f};
+    if (i < ntris) {
+        const float4 a = tris[3ull * i + 1], b = tris[3ull * i + 2];
+        const uint32_t li = tri_leaf[i];
+        if (li != kNone) link = links[li];
+        e1[0] = a.x; e1[1] = a.y; e1[2] = a.z;
+        e2[0] = b.x; e2[1] = b.y; e2[2] = b.z;
+    }
+    fold_root_cones(link, e1, e2, agg, arrivals, cones);
 }
 
 // ---- refit, parallel over triangles --------------------------------------------------------
@@ -313,9 +390,12 @@ constexpr unsigned long long kKeyMaxIdentity = 0ull;
 // One thread per triangle: keys of its three vertices per axis, reduced over the warp's lanes of
 // the same leaf, then one atomicMin / atomicMax per (leaf, axis) from the segment's first lane.
 // keys: 6 per leaf slot (min x y z, max x y z), at the identity before the launch.
+// ROOTS: the hidden roots' cones too (fold_root_cones; the refresh before this launch left them out).
+template <bool ROOTS>
 __global__ void __launch_bounds__(256) k_refit_tris(const float4* __restrict__ verts, uint32_t ntris,
                                                     const uint32_t* __restrict__ tri_leaf,
-                                                    unsigned long long* keys) {
+                                                    unsigned long long* keys, const uint4* __restrict__ links,
+                                                    float4* agg, uint32_t* arrivals, float4* cones) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned lane = threadIdx.x & 31u;
     uint32_t slot = kNone;
@@ -325,6 +405,14 @@ __global__ void __launch_bounds__(256) k_refit_tris(const float4* __restrict__ v
         v[0] = verts[3ull * i];
         v[1] = verts[3ull * i + 1];
         v[2] = verts[3ull * i + 2];
+    }
+    if (ROOTS) {
+        uint4 link = make_uint4(kNone, 0u, 0u, 0u);
+        if (slot != kNone) link = links[slot];
+        // the subtractions of the triangle write
+        const float e1[3] = {fsub(v[1].x, v[0].x), fsub(v[1].y, v[0].y), fsub(v[1].z, v[0].z)};
+        const float e2[3] = {fsub(v[2].x, v[0].x), fsub(v[2].y, v[0].y), fsub(v[2].z, v[0].z)};
+        fold_root_cones(link, e1, e2, agg, arrivals, cones);
     }
     const uint32_t prev = __shfl_up_sync(kFull, slot, 1);
     const bool head = slot != kNone && (lane == 0u || prev != slot);
@@ -1288,7 +1376,7 @@ inline unsigned grid_for(uint32_t n, int block) { return (unsigned)((n + block -
 
 }  // namespace
 
-cudaError_t launch_write_tris(bvhgpu_ctx* ctx, DeviceBlas& b, const float* d_tris9, cudaStream_t s) {
+cudaError_t launch_write_tris(bvhgpu_ctx* ctx, DeviceBlas& b, const float* d_tris9, cudaStream_t s, uint32_t* decide) {
     if (b.ntris == 0) return cudaSuccess;
     LaunchScope scope(ctx, BVHGPU_K_OTHER, s);
     k_write_tris<<<grid_for(b.ntris, 256), 256, 0, s>>>(d_tris9, b.ntris, b.tris, b.verts,
@@ -1296,23 +1384,30 @@ cudaError_t launch_write_tris(bvhgpu_ctx* ctx, DeviceBlas& b, const float* d_tri
     g_launches++;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return launch_hidden_refresh(ctx, b, s);
+    return launch_hidden_refresh(ctx, b, s, false, decide);
 }
 
-cudaError_t launch_hidden_refresh(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s) {
+cudaError_t launch_hidden_refresh(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s, bool refit_follows, uint32_t* decide) {
     if (b.nhid == 0) return cudaSuccess;
     LaunchScope scope(ctx, BVHGPU_K_OTHER, s);
     k_hidden_refresh<<<grid_for(4u * b.nhid, 256), 256, 0, s>>>(
         b.tris, b.hx + hidden_table_u2(b.ntris), pairs_in_order(b.ntris), reinterpret_cast<float4*>(b.pairs),
-        b.nodes + 2ull * b.nodes_used, b.nhid, b.hup, b.hagg, b.harrivals, b.cones);
+        b.nodes + 2ull * b.nodes_used, b.nhid, b.hup, b.hagg, b.harrivals, b.cones, b.measured_roots, decide);
     g_launches++;
+    if (b.measured_roots && !refit_follows) {
+        k_hidden_root_cones<<<grid_for(b.ntris, 256), 256, 0, s>>>(b.tris, b.ntris, b.tri_leaf, b.hup + b.nhid, b.hagg,
+                                                                  b.harrivals, b.cones);
+        g_launches++;
+    }
     return cudaGetLastError();
 }
 
-cudaError_t launch_refit(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s) {
+cudaError_t launch_refit(bvhgpu_ctx* ctx, DeviceBlas& b, cudaStream_t s, bool after_refresh) {
     if (b.nleaves == 0) return cudaSuccess;
     LaunchScope scope(ctx, BVHGPU_K_REFIT, s);
-    k_refit_tris<<<grid_for(b.ntris, 256), 256, 0, s>>>(b.verts, b.ntris, b.tri_leaf, b.leaf_keys);
+    auto* tris = after_refresh && b.measured_roots ? k_refit_tris<true> : k_refit_tris<false>;
+    tris<<<grid_for(b.ntris, 256), 256, 0, s>>>(b.verts, b.ntris, b.tri_leaf, b.leaf_keys, b.hup + b.nhid, b.hagg, b.harrivals,
+                                                b.cones);
     k_refit_leaves<<<grid_for(b.nleaves, kBlock), kBlock, 0, s>>>(b.nodes, b.verts, b.leaves, b.nleaves, b.parent,
                                                                   b.counters, b.leaf_keys);
     g_launches += 2;

@@ -39,6 +39,7 @@ struct PlanNode {
 struct PlanCounters {
     uint32_t nhid, nnext, ncones, largest;  // hidden nodes so far, next level's nodes, cones, its largest range
     uint32_t nhp;                           // hidden pairs
+    uint32_t decide;                        // the first refresh's word (launch_hidden_refresh)
 };
 
 __device__ __forceinline__ uint32_t rank_of(float f) {  // order-preserving
@@ -400,12 +401,21 @@ __global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* __restrict__ sums,
     if (threadIdx.x == 0) ctr->nhp = base;
 }
 
-// One thread per hidden node: its record (box zero until the refresh) and a leaf's pair slots.
+// One thread per hidden node: its record (box zero until the refresh) and a leaf's pair slots; one per
+// reference leaf: its link for the roots' cones (fold_root_cones, kernels_scene.cu).
 __global__ void k_plan_finish(const uint2* __restrict__ meta, const uint2* __restrict__ range, uint32_t nhid,
                               const uint32_t* __restrict__ ids, const uint32_t* __restrict__ pair_at,
                               const uint32_t* __restrict__ sums, uint32_t p0, float4* __restrict__ nodes,
-                              uint2* __restrict__ slots) {
+                              uint2* __restrict__ slots, const float4* __restrict__ ref_nodes, uint32_t nodes_used,
+                              const uint32_t* __restrict__ leaves, uint32_t nleaves, const uint2* __restrict__ table,
+                              uint4* __restrict__ links) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nleaves) {
+        const float4* N = ref_nodes + 2ull * leaves[i];
+        const uint2 e = table[__float_as_uint(N[0].w)];
+        links[i] = e.x ? make_uint4(e.x - nodes_used, e.y & kConeMask, __float_as_uint(N[1].w), 0u)
+                       : make_uint4(kNoRefresh, 0u, 0u, 0u);
+    }
     if (i >= nhid) return;
     const uint2 r = range[i];
     uint2 m = meta[i];
@@ -471,7 +481,8 @@ cudaError_t plan_hidden(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t node
     plan.up = reinterpret_cast<uint4*>(W + o_up);
     plan.table = reinterpret_cast<uint2*>(W + o_table);
     auto* ctr = reinterpret_cast<PlanCounters*>(W + o_ctr);
-    PlanCounters h = {0u, (uint32_t)roots.size(), (uint32_t)roots.size(), largest, 0u};
+    PlanCounters h = {0u, (uint32_t)roots.size(), (uint32_t)roots.size(), largest, 0u, 0u};
+    plan.decide = &ctr->decide;
     if ((e = cudaMemcpyAsync(q[0], roots.data(), sizeof(PlanNode) * roots.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(ctr, &h, sizeof(h), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(plan.table, 0, 8ull * plan.table_u2, s)) != cudaSuccess)
@@ -517,9 +528,10 @@ cudaError_t finish_hidden(bvhgpu_ctx* ctx, const HiddenPlan& plan, DeviceBlas& b
         (e = cudaMemcpyAsync(b.hup, plan.up, 16ull * plan.nhid, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
         return e;
     LaunchScope scope(ctx, BVHGPU_K_OTHER, s);
-    k_plan_finish<<<grid_for(plan.nhid, 128), 128, 0, s>>>(plan.meta, plan.range, plan.nhid, plan.ids, plan.pair_at, plan.sums,
-                                                           pairs_in_order(b.ntris), b.nodes + 2ull * b.nodes_used,
-                                                           b.hx + plan.table_u2);
+    k_plan_finish<<<grid_for(std::max(plan.nhid, b.nleaves), 128), 128, 0, s>>>(
+        plan.meta, plan.range, plan.nhid, plan.ids, plan.pair_at, plan.sums, pairs_in_order(b.ntris),
+        b.nodes + 2ull * b.nodes_used, b.hx + plan.table_u2, b.nodes, b.nodes_used, b.leaves, b.nleaves, plan.table,
+        b.hup + plan.nhid);
     g_launches++;
     return cudaGetLastError();
 }

@@ -45,3 +45,59 @@ def test_degenerate_and_non_finite_triangles(ctx):
         blas.update_vertices(good)
         check_hidden_records(blas, good)
     blas.free()
+
+
+def least_cosine(e1, e2, axis):
+    """cone_terms (cull.cuh) restated in float32, operation by operation: the least lower bound of
+    |N . A| / (|N| |A|) over the triangles."""
+    f = np.float32
+    u0 = f(2.0 ** -24)
+    e1, e2 = e1.T, e2.T
+    n, en = [], []
+    for i, j in ((1, 2), (2, 0), (0, 1)):
+        a, b = e1[i] * e2[j], e1[j] * e2[i]
+        n.append(a - b)
+        en.append(f(3) * u0 * (np.abs(a) + np.abs(b)))
+    dot = err = nn = n_err = np.zeros(e1.shape[1], f)
+    aa = f(0)
+    for i in range(3):
+        dot = dot + n[i] * axis[i]
+        err = err + (en[i] + f(4) * u0 * np.abs(n[i])) * np.abs(axis[i])
+        nn = nn + n[i] * n[i]
+        n_err = n_err + en[i]
+        aa = aa + axis[i] * axis[i]
+    nlen, alen = np.sqrt(nn), np.sqrt(aa)
+    one = f(1)
+    num = np.abs(dot) - err
+    den = (nlen * (one + f(8) * u0) + n_err) * alen * (one + f(8) * u0)
+    n_lo = (nlen * (one - f(8) * u0) - n_err) * (one - f(4) * u0)
+    return np.where((num > 0) & (den > 0) & (n_lo > 0), num / den * (one - f(8) * u0), f(-1)).min()
+
+
+@pytest.mark.parametrize("n", [16, 17, 127, 129, 513, 5000, 20480])
+@pytest.mark.parametrize("one", [True, False])
+def test_root_cones_are_as_narrow_as_their_triangles(ctx, n, one):
+    """In a large model a hidden root's cone is the one its triangles' normals span around its axis, bit for
+    bit, after the upload and after updates: leaves of one root, of many, and warps that hold several."""
+    tris = (scenes.displaced_icosphere(5, 2).triangles()[:n] * np.float32(100)).copy()
+    bvh = one_leaf_bvh(tris) if one else bt.BvhBuilder().build_for(tris)
+    blas = ctx.upload_blas(bvh, tris)
+    leaves = [x for x in bvh.nodes[:bvh.nodes_used] if x["primitive_count"] >= 16]
+    for k in range(3):
+        if k:
+            tris = (tris * np.float32([1.0, 1.0 + 0.2 * k, 1.0] * 3)).astype(np.float32)
+            blas.update_vertices(tris)
+        hd = blas.hidden_download()
+        v = tris.reshape(-1, 3, 3)
+        e1, e2 = v[:, 1] - v[:, 0], v[:, 2] - v[:, 0]
+        seen = 0
+        for leaf in leaves:
+            first, count = int(leaf["left_first"]), int(leaf["primitive_count"])
+            cone = hd["cones"][int(hd["table"][first, 1]) & 0x0FFFFFFF]
+            if cone[3] <= 0:
+                assert not cone[:3].any()  # some normals lie square to the axis
+                continue
+            assert cone[3] == least_cosine(e1[first:first + count], e2[first:first + count], cone[:3])
+            seen += 1
+        assert seen >= (len(leaves) + 1) // 2 or (one and n > 100)
+    blas.free()
