@@ -1471,7 +1471,7 @@ cudaError_t launch_trace_scene(bvhgpu_ctx* ctx, DeviceScene& sc, const float4* r
     SceneData sd = scene_data(ctx, sc, &depth);
     LaunchScope scope(ctx, BVHGPU_K_TRACE_SCENE, s);
     const Variant v = resolve(ctx->tune[BVHGPU_K_TRACE_SCENE], depth);
-    if (n <= wide_rays(ctx, BVHGPU_K_TRACE_SCENE, sc.instanced_tris)) {
+    if (n <= wide_rays(ctx, BVHGPU_K_TRACE_SCENE, sc)) {
         k_trace_scene_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(sd, rays, n, static_cast<GHit*>(hits), v.pol,
                                                                                ctx->d_err);
         g_launches++;
@@ -1499,7 +1499,7 @@ cudaError_t launch_render_scene(bvhgpu_ctx* ctx, DeviceScene& sc, const bvhgpu_c
     const unsigned tiles = (unsigned)(((w + 7) / 8) * ((h + 7) / 8));
     LaunchScope scope(ctx, BVHGPU_K_RENDER, s);
     const uint64_t px = (uint64_t)w * (uint64_t)h;
-    if (px <= wide_rays(ctx, BVHGPU_K_TRACE_SCENE, sc.instanced_tris)) {
+    if (px <= wide_rays(ctx, BVHGPU_K_TRACE_SCENE, sc)) {
         k_render_scene_wide<<<grid_for((uint32_t)px, kWideWarps), 32 * kWideWarps, 0, s>>>(sd, P, d_shade, sc.xf, lookup, d_rgba,
                                                                                            pol, ctx->d_err);
         g_launches++;
@@ -1524,7 +1524,7 @@ cudaError_t launch_scene_bounce(bvhgpu_ctx* ctx, DeviceScene& sc, const float4* 
     uint32_t depth = 1;
     SceneData sd = scene_data(ctx, sc, &depth);
     const Variant v = resolve(ctx->tune[BVHGPU_K_SCENE_BOUNCE], depth);
-    if (n <= wide_rays(ctx, BVHGPU_K_SCENE_BOUNCE, sc.instanced_tris)) {
+    if (n <= wide_rays(ctx, BVHGPU_K_SCENE_BOUNCE, sc)) {
         LaunchScope scope(ctx, BVHGPU_K_SCENE_BOUNCE, s);
         k_scene_bounce_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(sd, rays, n, seed, static_cast<GHit*>(hits0),
                                                                                 static_cast<GHit*>(hits1), v.pol, ctx->d_err);

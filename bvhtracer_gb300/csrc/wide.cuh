@@ -11,6 +11,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.hpp"
 
@@ -219,11 +221,21 @@ __device__ __forceinline__ bool wide_blas(const GBlas& g, LaneRay& r, LeafPolicy
 //  scene of 3 small objects               25 | 23 | 23 | 23 -> 15 | 19 | 27 | 44
 //  scene of 1,000 objects                 236 | 257 | 277 | 312 -> 47 | 72 | 126 | 226
 //  scene bounce, 1,000 objects            541 | 548 | 574 | 636 -> 86 | 125 | 217 | 399
+//  scene of 1,000 objects of 80 triangles 104 | 104 | 109 | 123 -> 52 | 87 | 142 | 259
+//  its bounce                             282 | 295 | 303 | 314 -> 87 | 140 | 242 | 444
 // `small`: the line for fewer than 4,096 triangles (all objects' together); 8,192 where a ray's work is
 // one closest hit in one small mesh.
 inline uint32_t wide_rays(const bvhgpu_ctx* ctx, int kernel, uint64_t ntris, uint32_t small = 16384u) {
     if (!default_tune(ctx->tune[kernel], kernel)) return 0u;
     return ntris < 4096u ? small : ntris < 65536u ? 32768u : 65536u;
+}
+
+// The line of a scene.  Where many objects are tiny a ray's walk is mostly TLAS, which the warp follows no
+// faster than a thread: the line stays at 16,384, with a bounce at 32,768.
+inline uint32_t wide_rays(const bvhgpu_ctx* ctx, int kernel, const DeviceScene& sc) {
+    const uint32_t n = wide_rays(ctx, kernel, sc.instanced_tris);
+    if (sc.nobjects < 128u || sc.instanced_tris >= 200ull * sc.nobjects) return n;
+    return std::min(n, kernel == BVHGPU_K_SCENE_BOUNCE ? 32768u : 16384u);
 }
 
 }  // namespace bvhgpu

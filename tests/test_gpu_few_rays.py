@@ -195,3 +195,36 @@ def test_default_and_set_configs_agree(ctx):
         assert blas.intersect(rays).tobytes() == a.tobytes()
     finally:
         ctx.tune_set(bt.K_TRACE_BLAS, **saved)
+
+
+@pytest.mark.parametrize("n", [16384, 16385, 32768, 32769, 65536])
+def test_scene_of_many_tiny_objects(ctx, n):
+    """Many objects of 80 triangles: hits and bounces on both sides of their own lines, the closest hits
+    against the oracle and the bounces against a set config."""
+    tris = scenes.displaced_icosphere(1, 6).triangles().copy()
+    bvh = bt.BvhBuilder().build_for(tris)
+    blas = ctx.upload_blas(bvh, tris)
+    k = 900
+    rng = np.random.default_rng(k)
+    xf = np.tile(np.eye(4, dtype=np.float32).reshape(1, 16), (k, 1))
+    inv = xf.copy()
+    xf[:, 12:15] = rng.uniform(-12, 12, (k, 3))
+    inv[:, 12:15] = -xf[:, 12:15]
+    sc = ctx.scene([blas] * k, xf, inv)
+    tl, used = sc.download_tlas()
+    sa = orc.SceneArrays([(bvh.nodes[:bvh.nodes_used], bvh.nodes_used, tris)], np.zeros(k, np.int64), inv)
+    rays = np.concatenate([scenes.look_at_rays(128, 128, (0, 1.0, -40.0), (0, 0, 0), 45.0), scenes.sphere_rays(n, 3, box=14.0)])[:n]
+    d_rays, d0, d1 = ctx.to_device(rays), ctx.device_buffer(20 * n), ctx.device_buffer(20 * n)
+    saved = ctx.tune_get(bt.K_SCENE_BOUNCE)
+    out = []
+    try:
+        for cfg in ({}, {"hidden": 500}):
+            ctx.tune_set(bt.K_SCENE_BOUNCE, **cfg)
+            sc.trace_bounce_async(d_rays, n, 5, d0, d1)
+            out.append(d0.download(np.zeros(n, bt.HIT)).tobytes() + d1.download(np.zeros(n, bt.HIT)).tobytes())
+    finally:
+        ctx.tune_set(bt.K_SCENE_BOUNCE, **saved)
+    assert out[0] == out[1]
+    assert sc.intersect(rays).tobytes() == orc.scene_intersect(tl, used, sa, rays, threads=8).tobytes()
+    sc.free()
+    blas.free()
