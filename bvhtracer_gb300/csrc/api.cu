@@ -576,6 +576,7 @@ int bvhgpu_set_deadline(bvhgpu_ctx* ctx, uint64_t ns) {
     if (ctx->capturing) return fail(ctx, BVHGPU_ERR_INVALID_ARG, "set_deadline: not allowed during capture");
     CK(cudaMemcpyAsync(ctx->d_err + 2, &ns, sizeof(ns), cudaMemcpyHostToDevice, ctx->stream), "deadline");
     CK(cudaStreamSynchronize(ctx->stream), "stream synchronize");
+    ctx->deadline_ns = ns;
     return BVHGPU_OK;
 }
 

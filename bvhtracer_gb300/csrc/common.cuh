@@ -28,16 +28,33 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// A persistent launch's time budget (bvhgpu_set_deadline), kept in the two words after the
+// A launch's time budget (bvhgpu_set_deadline), kept in the two words after the
 // context's error word (0: none).  A warp stops taking and tracing rays once its launch has run
 // longer, raises kErrDeadline and leaves: no wait, so an expired launch ends promptly, and the host
 // reports the launch's outputs as incomplete.
 struct Deadline {
     unsigned long long end;  // globaltimer value at which the warp stops; 0: no deadline
-    __device__ __forceinline__ void start(const uint32_t* err) {
+    // For launches whose warps are all resident: they start together.
+    __device__ __forceinline__ void start(const uint32_t* err) { from(err, global_ns()); }
+    // For launches whose warps start one after another: from the launch's first warp on, whose start
+    // `first` keeps (zero before the launch; null: no deadline).
+    __device__ __forceinline__ void start(const uint32_t* err, unsigned long long* first) {
+        end = 0ull;
+        if (first == nullptr) return;
+        unsigned long long t = 0ull;
+        if ((threadIdx.x & 31u) == 0u) {
+            t = *static_cast<volatile unsigned long long*>(first);
+            if (t == 0ull) {
+                const unsigned long long now = global_ns();
+                t = atomicCAS(first, 0ull, now);
+                if (t == 0ull) t = now;
+            }
+        }
+        from(err, __shfl_sync(0xFFFFFFFFu, t, 0));
+    }
+    __device__ __forceinline__ void from(const uint32_t* err, unsigned long long t) {
         const unsigned long long budget = *reinterpret_cast<const volatile unsigned long long*>(err + 2);
-        const unsigned long long now = global_ns();
-        end = budget == 0ull ? 0ull : budget > ~0ull - now ? ~0ull : now + budget;  // saturating
+        end = budget == 0ull ? 0ull : budget > ~0ull - t ? ~0ull : t + budget;  // saturating
     }
     // Warp-uniform: lane 0's clock decides.
     __device__ __forceinline__ bool expired(uint32_t* err) const {

@@ -147,6 +147,7 @@ struct bvhgpu_ctx {
     cudaStream_t stream = nullptr;
     void* host_word = nullptr;  // 64 bytes of pinned host memory for small results
     uint32_t* d_err = nullptr;       // device error flags
+    uint64_t deadline_ns = 0;        // the launch deadline on the device beside them (bvhgpu_set_deadline)
     uint32_t* d_scratch = nullptr;   // small device scratch: queue counters etc. (64 words)
     void* l2_flush = nullptr;
     size_t l2_flush_bytes = 0;

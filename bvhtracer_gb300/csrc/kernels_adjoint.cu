@@ -260,12 +260,12 @@ __global__ void __launch_bounds__(32 * kWideWarps) k_lambert_forward_wide(GBlas 
                                                                           const float* __restrict__ verts,
                                                                           const float* __restrict__ vnormals, float3 light,
                                                                           float* __restrict__ image, GHit* __restrict__ hits,
-                                                                          LeafPolicy pol, uint32_t* err) {
+                                                                          LeafPolicy pol, uint32_t* err, unsigned long long* began) {
     __shared__ WideSmem smem[kWideWarps];
     const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
     if (i >= n) return;
     Deadline dl;
-    dl.start(err);
+    dl.start(err, began);
     LaneRay r;
     float3 o, d;
     float t0;
@@ -385,9 +385,12 @@ cudaError_t launch_lambert_forward(bvhgpu_ctx* ctx, DeviceMesh& m, const DeviceB
     // kernel's launch config, and its refill threshold
     const Variant v = resolve(ctx->tune[BVHGPU_K_TRACE_BLAS], b.depth);
     if (n <= wide_rays(ctx, BVHGPU_K_TRACE_BLAS, b.ntris)) {
+        unsigned long long* began;
+        cudaError_t e = launch_start(ctx, s, &began);
+        if (e != cudaSuccess) return e;
         LaunchScope scope(ctx, BVHGPU_K_LAMBERT_FORWARD, s);
         k_lambert_forward_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(
-            g, rays, n, m.faces, m.verts, m.vnormals, L, image, static_cast<GHit*>(hits), v.pol, ctx->d_err);
+            g, rays, n, m.faces, m.verts, m.vnormals, L, image, static_cast<GHit*>(hits), v.pol, ctx->d_err, began);
         g_launches++;
         return cudaGetLastError();
     }

@@ -1168,14 +1168,15 @@ __global__ void __launch_bounds__(32 * kWideWarps) k_render_scene_wide(SceneData
 
 __global__ void __launch_bounds__(32 * kWideWarps) k_scene_bounce_wide(SceneData sd, const float4* __restrict__ rays, uint32_t n,
                                                                        uint32_t seed, GHit* __restrict__ hits0,
-                                                                       GHit* __restrict__ hits1, LeafPolicy pol, uint32_t* err) {
+                                                                       GHit* __restrict__ hits1, LeafPolicy pol, uint32_t* err,
+                                                                       unsigned long long* began) {
     __shared__ WideSceneSmem smem[kWideWarps];
     WideSceneSmem& sm = smem[threadIdx.x >> 5];
     const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
     const bool first = (threadIdx.x & 31u) == 0u;
     if (i >= n) return;
     Deadline deadline;
-    deadline.start(err);
+    deadline.start(err, began);
     LaneRay r;
     float3 o, d;
     float t0;
@@ -1525,9 +1526,12 @@ cudaError_t launch_scene_bounce(bvhgpu_ctx* ctx, DeviceScene& sc, const float4* 
     SceneData sd = scene_data(ctx, sc, &depth);
     const Variant v = resolve(ctx->tune[BVHGPU_K_SCENE_BOUNCE], depth);
     if (n <= wide_rays(ctx, BVHGPU_K_SCENE_BOUNCE, sc)) {
+        unsigned long long* began;
+        const cudaError_t e = launch_start(ctx, s, &began);
+        if (e != cudaSuccess) return e;
         LaunchScope scope(ctx, BVHGPU_K_SCENE_BOUNCE, s);
         k_scene_bounce_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(sd, rays, n, seed, static_cast<GHit*>(hits0),
-                                                                                static_cast<GHit*>(hits1), v.pol, ctx->d_err);
+                                                                                static_cast<GHit*>(hits1), v.pol, ctx->d_err, began);
         g_launches++;
         return cudaGetLastError();
     }

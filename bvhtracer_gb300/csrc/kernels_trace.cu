@@ -122,14 +122,15 @@ __global__ void __launch_bounds__(32 * kWideWarps) k_trace_wide(GBlas g, const f
 __global__ void __launch_bounds__(32 * kWideWarps) k_bounce_wide(GBlas b, const float4* __restrict__ rays, uint32_t n,
                                                                  uint32_t seed, GHit* __restrict__ hits0,
                                                                  GHit* __restrict__ hits1, LeafPolicy pol, uint32_t key0,
-                                                                 uint32_t* hit_count, uint32_t* err) {
+                                                                 uint32_t* hit_count, uint32_t* err,
+                                                                 unsigned long long* began) {
     __shared__ WideSmem smem[kWideWarps];
     WideSmem& sm = smem[threadIdx.x >> 5];
     const uint32_t i = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
     const bool first = (threadIdx.x & 31u) == 0u;
     if (i >= n) return;
     Deadline dl;
-    dl.start(err);
+    dl.start(err, began);
     LaneRay r;
     float3 o, d;
     float t0;
@@ -604,9 +605,13 @@ cudaError_t launch_bounce_persistent(bvhgpu_ctx* ctx, const DeviceBlas& b, const
     GBlas g = to_gblas(b);
     const Variant v = resolve(ctx->tune[BVHGPU_K_PERSISTENT_BOUNCE], b.depth);
     if (n <= wide_rays(ctx, BVHGPU_K_PERSISTENT_BOUNCE, b.ntris)) {
+        unsigned long long* began;
+        const cudaError_t e = launch_start(ctx, s, &began);
+        if (e != cudaSuccess) return e;
         LaunchScope scope(ctx, BVHGPU_K_PERSISTENT_BOUNCE, s);
         k_bounce_wide<<<grid_for(n, kWideWarps), 32 * kWideWarps, 0, s>>>(
-            g, rays, n, seed, static_cast<GHit*>(hits0), static_cast<GHit*>(hits1), v.pol, base, hit_count, ctx->d_err);
+            g, rays, n, seed, static_cast<GHit*>(hits0), static_cast<GHit*>(hits1), v.pol, base, hit_count, ctx->d_err,
+            began);
         g_launches++;
         return cudaGetLastError();
     }

@@ -230,6 +230,17 @@ inline uint32_t wide_rays(const bvhgpu_ctx* ctx, int kernel, uint64_t ntris, uin
     return ntris < 4096u ? small : ntris < 65536u ? 32768u : 65536u;
 }
 
+// The word in which a warp-per-ray launch keeps its start (Deadline::start), zeroed on the stream, or null where
+// no deadline can apply: none set, and no capture whose replays may come under one.
+inline cudaError_t launch_start(bvhgpu_ctx* ctx, cudaStream_t s, unsigned long long** first) {
+    *first = nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    if (e != cudaSuccess || (ctx->deadline_ns == 0u && capture == cudaStreamCaptureStatusNone)) return e;
+    *first = reinterpret_cast<unsigned long long*>(ctx->d_scratch + 12);
+    return cudaMemsetAsync(*first, 0, sizeof(**first), s);
+}
+
 // The line of a scene.  Where many objects are tiny a ray's walk is mostly TLAS, which the warp follows no
 // faster than a thread: the line stays at 16,384, with a bounce at 32,768.
 inline uint32_t wide_rays(const bvhgpu_ctx* ctx, int kernel, const DeviceScene& sc) {

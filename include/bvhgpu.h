@@ -138,8 +138,8 @@ uint64_t bvhgpu_launch_count(void);
 int bvhgpu_sync(bvhgpu_ctx* ctx);
 bvhgpu_stream bvhgpu_get_stream(bvhgpu_ctx* ctx);
 /* A time budget for each persistent launch of this context (the single-BLAS bounce, batch, scene
- * bounce and Lambertian forward launches), in nanoseconds of the device clock from the start of
- * each of its warps; 0 (the default) means none.  A launch past it stops taking and tracing rays
+ * bounce and Lambertian forward launches, few rays or many), in nanoseconds of the device clock from
+ * the start of the launch; 0 (the default) means none.  A launch past it stops taking and tracing rays
  * and the next synchronising call (or bvhgpu_sync) returns BVHGPU_ERR_DEADLINE; that launch's
  * outputs are then incomplete, and the context stays usable.  For a serving caller that must
  * bound a frame's time; no reference counterpart (the reference has no time limit).  Applies to
