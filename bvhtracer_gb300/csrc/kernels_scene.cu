@@ -151,10 +151,11 @@ __device__ __forceinline__ float wider_cone(const float* a, const float* s, floa
 }
 
 // Whether the plain margin (leaf_cull) of a tree with bounds Q, B is too wide to walk it (2, the default limit)
-// already for rays from within 7 B of the origin: its cone alone then decides.  Below, the looser roots cost
-// nothing measurable, and the second pass over the triangles would (update of 20,480 triangles 25 -> 32 us).
+// already for rays from within 2 B of the origin: its cone alone then decides.  Below, the looser roots cost
+// nothing measurable, and the second pass over the triangles would (update of 20,480 triangles 25 -> 32 us,
+// with a refit 43 -> 46).
 __device__ __forceinline__ bool cones_decide(float Q, float B) {
-    const float w = 2.0f * 1.7320508f * 8.0f * B;  // W of a unit direction along the diagonal
+    const float w = 2.0f * 1.7320508f * 3.0f * B;  // W of a unit direction along the diagonal
     return !(8.0f * kCullUnit * w * Q + 28.0f * kCullUnit * 1.7320508f * 0.25f * Q * Q < 2.0f * 0.0001f);
 }
 
@@ -406,14 +407,6 @@ __global__ void __launch_bounds__(256) k_refit_tris(const float4* __restrict__ v
         v[1] = verts[3ull * i + 1];
         v[2] = verts[3ull * i + 2];
     }
-    if (ROOTS) {
-        uint4 link = make_uint4(kNone, 0u, 0u, 0u);
-        if (slot != kNone) link = links[slot];
-        // the subtractions of the triangle write
-        const float e1[3] = {fsub(v[1].x, v[0].x), fsub(v[1].y, v[0].y), fsub(v[1].z, v[0].z)};
-        const float e2[3] = {fsub(v[2].x, v[0].x), fsub(v[2].y, v[0].y), fsub(v[2].z, v[0].z)};
-        fold_root_cones(link, e1, e2, agg, arrivals, cones);
-    }
     const uint32_t prev = __shfl_up_sync(kFull, slot, 1);
     const bool head = slot != kNone && (lane == 0u || prev != slot);
 #pragma unroll
@@ -437,6 +430,14 @@ __global__ void __launch_bounds__(256) k_refit_tris(const float4* __restrict__ v
             if (kmin != kKeyMinIdentity) atomicMin(&keys[6ull * slot + axis], kmin);
             if (kmax != kKeyMaxIdentity) atomicMax(&keys[6ull * slot + 3 + axis], kmax);
         }
+    }
+    if (ROOTS) {
+        uint4 link = make_uint4(kNone, 0u, 0u, 0u);
+        if (slot != kNone) link = links[slot];
+        // the subtractions of the triangle write
+        const float e1[3] = {fsub(v[1].x, v[0].x), fsub(v[1].y, v[0].y), fsub(v[1].z, v[0].z)};
+        const float e2[3] = {fsub(v[2].x, v[0].x), fsub(v[2].y, v[0].y), fsub(v[2].z, v[0].z)};
+        fold_root_cones(link, e1, e2, agg, arrivals, cones);
     }
 }
 
