@@ -7,13 +7,13 @@
 //
 // The trees grow level by level, one block per 4-wide node: k_plan_split splits its range and both
 // halves (centroid bounds, bins and a stable partition, each a pass of the block over the range),
-// k_plan_scan numbers the children, k_plan_emit writes them and queues those to be split.  Node order
-// and tree shape depend on the triangles only.  The leaves' packed pairs are numbered at the end by a
-// prefix sum over the triangle positions.  Boxes and cones come from the refresh (k_hidden_refresh).
+// k_plan_scan numbers the children and writes them, or in a level of many nodes k_plan_emit, and queues
+// those to be split.  Node order and tree shape depend on the triangles only.  The leaves' packed pairs
+// are numbered at the end by a prefix sum over the triangle positions.  Boxes and cones come from the refresh (k_hidden_refresh).
 //
 // What bounds it: one block's passes over the largest range, then the launches of the levels (about
 // log4(largest leaf / 8)).  The same planning on one host core made a model of 81,920 triangles take
-// 28.1 ms to upload, now 0.96 ms; 20,000 triangles of a soup 6.9 -> 0.60 ms; 1,280 triangles 0.48 -> 0.24 ms.
+// 28.1 ms to upload, now 0.96 ms; 20,480 triangles 7.0 -> 0.73 ms; 1,280 triangles 0.49 -> 0.18 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,6 +29,7 @@ namespace {
 constexpr int kBins = 16;
 constexpr int kPlanThreads = 512;
 constexpr uint32_t kSahLevels = 16;  // 4-wide levels split by SAH; deeper ones in halves
+constexpr uint32_t kPlanSmall = 2048;  // triangles of a model whose levels are queued ahead
 
 struct PlanNode {
     uint32_t a, b;  // range of triangle positions
@@ -40,6 +41,7 @@ struct PlanCounters {
     uint32_t nhid, nnext, ncones, largest;  // hidden nodes so far, next level's nodes, cones, its largest range
     uint32_t nhp;                           // hidden pairs
     uint32_t decide;                        // the first refresh's word (launch_hidden_refresh)
+    uint32_t levels;                        // levels split so far
 };
 
 __device__ __forceinline__ uint32_t rank_of(float f) {  // order-preserving
@@ -236,8 +238,10 @@ __device__ uint32_t block_split(const uint32_t* in, uint32_t* out, uint32_t x, u
 
 // One block per node: its 2 to 4 ranges, res = {end of range 0, of range 1, of range 2, ranges}.
 __global__ void k_plan_split(const PlanNode* __restrict__ cur, uint32_t* ids, uint32_t* tmp, const float4* __restrict__ cen,
-                             const float4* __restrict__ lo, const float4* __restrict__ hi, int sah, uint4* __restrict__ res) {
+                             const float4* __restrict__ lo, const float4* __restrict__ hi, int sah, uint4* __restrict__ res,
+                             const PlanCounters* __restrict__ ctr) {
     __shared__ PlanSmem sm;
+    if (blockIdx.x >= ctr->nnext) return;
     const PlanNode nd = cur[blockIdx.x];
     const uint32_t m = block_split(ids, tmp, nd.a, nd.b, sah != 0, cen, lo, hi, sm);
     uint32_t r[4], k = 0u;
@@ -262,18 +266,60 @@ __device__ __forceinline__ void plan_ranges(const PlanNode& nd, uint4 s, uint32_
     r[s.w] = nd.b;
 }
 
-// One block: off[i] = {children, children to be split} before node i; the counters move on.
-__global__ void __launch_bounds__(1024) k_plan_scan(const PlanNode* __restrict__ cur, const uint4* __restrict__ res, uint32_t n,
-                                                    uint2* __restrict__ off, PlanCounters* ctr) {
+struct PlanOut {  // where a level's nodes go
+    uint32_t nodes_used;
+    PlanNode* next;
+    uint2 *meta, *range;
+    uint4* up;
+    uint32_t* np_at;
+    uint2* table;
+};
+
+// Node nd of a level that has nhid0 hidden nodes and ncones0 cones before it, o = {children, children to be
+// split} of the level's nodes before nd: its own record (or table entry), its children's links, the next
+// level's queue.
+__device__ __forceinline__ void plan_emit(const PlanNode& nd, uint4 s, uint2 o, uint32_t nhid0, uint32_t ncones0, const PlanOut& out) {
+    uint32_t r[5];
+    plan_ranges(nd, s, r);
+    const uint32_t li = nhid0 + o.x, k = s.w;
+    const uint2 own = make_uint2(out.nodes_used + li, kHiddenInterior | ((k - 1u) << kWideShift) | nd.cone);
+    if (nd.me == kNoRefresh)
+        out.table[nd.a] = own;
+    else
+        out.meta[nd.me] = own;
+    uint32_t q = o.y;
+    for (uint32_t c = 0; c < k; ++c) {
+        const uint32_t x = r[c], y = r[c + 1];
+        out.up[li + c] = make_uint4(li, k, nd.me, nd.cone);
+        if (y - x > kHiddenLeafTris) {
+            out.next[q] = PlanNode{x, y, li + c, ncones0 + q};
+            out.range[li + c] = make_uint2(0u, 0u);
+            ++q;
+        } else {
+            out.range[li + c] = make_uint2(x, y);
+            out.np_at[x] = (y - x + 1u) / 2u;
+        }
+    }
+}
+
+// One block numbers a level's children and moves the counters on.  EMIT: and writes its nodes; else
+// off[i] = {children, children to be split} before node i.
+template <bool EMIT>
+__global__ void __launch_bounds__(1024) k_plan_scan(const PlanNode* __restrict__ cur, const uint4* __restrict__ res,
+                                                    uint2* __restrict__ off, PlanOut out, PlanCounters* ctr) {
     __shared__ uint32_t wk[32], wi[32];
+    const uint32_t n = ctr->nnext, nhid0 = ctr->nhid, ncones0 = ctr->ncones;
+    if (n == 0u) return;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
     uint32_t base_k = 0u, base_i = 0u, largest = 0u;
     for (uint32_t j0 = 0; j0 < n; j0 += 1024u) {
         const uint32_t j = j0 + tid;
         uint32_t k = 0u, in = 0u;
+        PlanNode nd;
+        uint4 s;
         if (j < n) {
-            const PlanNode nd = cur[j];
-            const uint4 s = res[j];
+            nd = cur[j];
+            s = res[j];
             uint32_t r[5];
             plan_ranges(nd, s, r);
             k = s.w;
@@ -308,7 +354,13 @@ __global__ void __launch_bounds__(1024) k_plan_scan(const PlanNode* __restrict__
             tk += wk[q];
             ti += wi[q];
         }
-        if (j < n) off[j] = make_uint2(base_k + bk + sk - k, base_i + bi + si - in);
+        if (j < n) {
+            const uint2 o = make_uint2(base_k + bk + sk - k, base_i + bi + si - in);
+            if (EMIT)
+                plan_emit(nd, s, o, nhid0, ncones0, out);
+            else
+                off[j] = o;
+        }
         base_k += tk;
         base_i += ti;
     }
@@ -320,46 +372,22 @@ __global__ void __launch_bounds__(1024) k_plan_scan(const PlanNode* __restrict__
         for (int q = 1; q < 32; ++q) wk[0] = max(wk[0], wk[q]);
         ctr->largest = wk[0];
         ctr->nnext = base_i;
-        ctr->nhid += base_k;
-        ctr->ncones += base_i;
+        ctr->nhid = nhid0 + base_k;
+        ctr->ncones = ncones0 + base_i;
+        ctr->levels += 1u;
     }
 }
 
-// One thread per node: its own record (or table entry), its children's links, the next level's queue.
+// One thread per node of a level of n, after its scan.
 __global__ void k_plan_emit(const PlanNode* __restrict__ cur, const uint4* __restrict__ res, uint32_t n,
-                            const uint2* __restrict__ off, uint32_t nhid0, uint32_t ncones0, uint32_t nodes_used,
-                            PlanNode* __restrict__ next, uint2* __restrict__ meta, uint2* __restrict__ range,
-                            uint4* __restrict__ up, uint32_t* __restrict__ np_at, uint2* __restrict__ table) {
+                            const uint2* __restrict__ off, uint32_t nhid0, uint32_t ncones0, PlanOut out) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const PlanNode nd = cur[j];
-    const uint4 s = res[j];
-    const uint2 o = off[j];
-    uint32_t r[5];
-    plan_ranges(nd, s, r);
-    const uint32_t li = nhid0 + o.x, k = s.w;
-    const uint2 own = make_uint2(nodes_used + li, kHiddenInterior | ((k - 1u) << kWideShift) | nd.cone);
-    if (nd.me == kNoRefresh)
-        table[nd.a] = own;
-    else
-        meta[nd.me] = own;
-    uint32_t q = o.y;
-    for (uint32_t c = 0; c < k; ++c) {
-        const uint32_t x = r[c], y = r[c + 1];
-        up[li + c] = make_uint4(li, k, nd.me, nd.cone);
-        if (y - x > kHiddenLeafTris) {
-            next[q] = PlanNode{x, y, li + c, ncones0 + q};
-            range[li + c] = make_uint2(0u, 0u);
-            ++q;
-        } else {
-            range[li + c] = make_uint2(x, y);
-            np_at[x] = (y - x + 1u) / 2u;
-        }
-    }
+    if (j < n) plan_emit(cur[j], res[j], off[j], nhid0, ncones0, out);
 }
 
-// Exclusive prefix sum of v[0, n): tiles of 1,024, then the tiles' sums, then the offsets.
-__global__ void __launch_bounds__(1024) k_scan_tiles(uint32_t* __restrict__ v, uint32_t n, uint32_t* __restrict__ sums) {
+// Exclusive prefix sum of v[0, n) into out: tiles of 1,024, then the tiles' sums.
+__global__ void __launch_bounds__(1024) k_scan_tiles(const uint32_t* __restrict__ v, uint32_t n, uint32_t* __restrict__ out,
+                                                     uint32_t* __restrict__ sums) {
     __shared__ uint32_t ws[32];
     const uint32_t i = blockIdx.x * 1024u + threadIdx.x, lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const uint32_t x = i < n ? v[i] : 0u;
@@ -372,7 +400,7 @@ __global__ void __launch_bounds__(1024) k_scan_tiles(uint32_t* __restrict__ v, u
     __syncthreads();
     uint32_t before = 0u;
     for (uint32_t q = 0; q < w; ++q) before += ws[q];
-    if (i < n) v[i] = before + s - x;
+    if (i < n) out[i] = before + s - x;
     if (threadIdx.x == 1023u) sums[blockIdx.x] = before + s;
 }
 __global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* __restrict__ sums, uint32_t n, PlanCounters* ctr) {
@@ -401,15 +429,17 @@ __global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* __restrict__ sums,
     if (threadIdx.x == 0) ctr->nhp = base;
 }
 
-// One thread per hidden node: its record (box zero until the refresh) and a leaf's pair slots; one per
-// reference leaf: its link for the roots' cones (fold_root_cones, kernels_scene.cu).
-__global__ void k_plan_finish(const uint2* __restrict__ meta, const uint2* __restrict__ range, uint32_t nhid,
-                              const uint32_t* __restrict__ ids, const uint32_t* __restrict__ pair_at,
+// One thread per table entry; per hidden node: its record (box zero until the refresh), its links and a leaf's
+// pair slots; per reference leaf: its link for the roots' cones (fold_root_cones, kernels_scene.cu).
+__global__ void k_plan_finish(const uint2* __restrict__ meta, const uint2* __restrict__ range, const uint4* __restrict__ up,
+                              uint32_t nhid, const uint32_t* __restrict__ ids, const uint32_t* __restrict__ pair_at,
                               const uint32_t* __restrict__ sums, uint32_t p0, float4* __restrict__ nodes,
-                              uint2* __restrict__ slots, const float4* __restrict__ ref_nodes, uint32_t nodes_used,
-                              const uint32_t* __restrict__ leaves, uint32_t nleaves, const uint2* __restrict__ table,
-                              uint4* __restrict__ links) {
+                              uint4* __restrict__ hup, uint2* __restrict__ slots, const float4* __restrict__ ref_nodes,
+                              uint32_t nodes_used, const uint32_t* __restrict__ leaves, uint32_t nleaves,
+                              const uint2* __restrict__ table, uint32_t table_u2, uint2* __restrict__ hx) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < table_u2) hx[i] = table[i];
+    uint4* links = hup + nhid;
     if (i < nleaves) {
         const float4* N = ref_nodes + 2ull * leaves[i];
         const uint2 e = table[__float_as_uint(N[0].w)];
@@ -417,6 +447,7 @@ __global__ void k_plan_finish(const uint2* __restrict__ meta, const uint2* __res
                        : make_uint4(kNoRefresh, 0u, 0u, 0u);
     }
     if (i >= nhid) return;
+    hup[i] = up[i];
     const uint2 r = range[i];
     uint2 m = meta[i];
     if (r.x != r.y) {
@@ -457,21 +488,27 @@ cudaError_t plan_hidden(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t node
         return at;
     };
     const size_t o_cen = part(16ull * ntris), o_lo = part(16ull * ntris), o_hi = part(16ull * ntris), o_ids = part(4ull * ntris),
-                 o_tmp = part(4ull * ntris), o_np = part(4ull * ntris), o_sums = part(4ull * tiles),
+                 o_tmp = part(4ull * ntris), o_np = part(4ull * ntris), o_at = part(4ull * ntris), o_sums = part(4ull * tiles),
                  o_q0 = part(sizeof(PlanNode) * max_level), o_q1 = part(sizeof(PlanNode) * max_level),
                  o_res = part(16ull * max_level), o_off = part(8ull * max_level), o_meta = part(8ull * max_nodes),
                  o_range = part(8ull * max_nodes), o_ctr = part(sizeof(PlanCounters));
     plan.table_u2 = hidden_table_u2(ntris);
     const size_t o_up = part(16ull * max_nodes), o_table = part(8ull * plan.table_u2);
-    cudaError_t e = cudaMalloc(&plan.work, bytes);
-    if (e != cudaSuccess) return e;
-    char* W = static_cast<char*>(plan.work);
+    cudaError_t e = cudaSuccess;
+    char* W;
+    if (bytes <= ctx->stage_out_bytes) {
+        W = static_cast<char*>(ctx->stage_out);  // the context's own staging memory, free between calls
+    } else {
+        if ((e = cudaMalloc(&plan.work, bytes)) != cudaSuccess) return e;
+        W = static_cast<char*>(plan.work);
+    }
     auto* cen = reinterpret_cast<float4*>(W + o_cen);
     auto* lo = reinterpret_cast<float4*>(W + o_lo);
     auto* hi = reinterpret_cast<float4*>(W + o_hi);
     plan.ids = reinterpret_cast<uint32_t*>(W + o_ids);
     auto* tmp = reinterpret_cast<uint32_t*>(W + o_tmp);
-    plan.pair_at = reinterpret_cast<uint32_t*>(W + o_np);
+    auto* np_at = reinterpret_cast<uint32_t*>(W + o_np);
+    plan.pair_at = reinterpret_cast<uint32_t*>(W + o_at);
     plan.sums = reinterpret_cast<uint32_t*>(W + o_sums);
     PlanNode* q[2] = {reinterpret_cast<PlanNode*>(W + o_q0), reinterpret_cast<PlanNode*>(W + o_q1)};
     auto* res = reinterpret_cast<uint4*>(W + o_res);
@@ -481,57 +518,75 @@ cudaError_t plan_hidden(bvhgpu_ctx* ctx, const bvhgpu_node* nodes, uint32_t node
     plan.up = reinterpret_cast<uint4*>(W + o_up);
     plan.table = reinterpret_cast<uint2*>(W + o_table);
     auto* ctr = reinterpret_cast<PlanCounters*>(W + o_ctr);
-    PlanCounters h = {0u, (uint32_t)roots.size(), (uint32_t)roots.size(), largest, 0u, 0u};
+    PlanCounters h = {0u, (uint32_t)roots.size(), (uint32_t)roots.size(), largest, 0u, 0u, 0u};
     plan.decide = &ctr->decide;
     if ((e = cudaMemcpyAsync(q[0], roots.data(), sizeof(PlanNode) * roots.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(ctr, &h, sizeof(h), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(plan.table, 0, 8ull * plan.table_u2, s)) != cudaSuccess)
         return e;
     LaunchScope scope(ctx, BVHGPU_K_OTHER, s);
-    k_plan_info<<<grid_for(ntris, 256), 256, 0, s>>>(d_tris9, ntris, cen, lo, hi, plan.ids, plan.pair_at);
+    k_plan_info<<<grid_for(ntris, 256), 256, 0, s>>>(d_tris9, ntris, cen, lo, hi, plan.ids, np_at);
     g_launches++;
-    uint32_t level = 0;
+    // Small models: the levels that a balanced tree has, and one more, are queued at once, their launches
+    // sized by what a level can hold, and the pairs numbered behind them, with one wait for it all: upload of
+    // one leaf of 100 triangles 230 -> 177 us (planned on the host 182), of 1,280 triangles 325 -> 230.
+    const bool small = ntris <= kPlanSmall;
+    uint32_t level = 0, most = h.nnext, ahead = 1;
+    if (small)
+        for (uint32_t reach = kHiddenLeafTris; reach < largest; reach *= 4u) ++ahead;
     while (h.nnext != 0u) {
-        const uint32_t n = h.nnext, nhid0 = h.nhid, ncones0 = h.ncones;
-        PlanNode* cur = q[level & 1u];
-        // small ranges: one triangle or two a thread
-        const int threads = h.largest > 512u ? kPlanThreads : h.largest > 128u ? 128 : 64;
-        k_plan_split<<<n, threads, 0, s>>>(cur, plan.ids, tmp, cen, lo, hi, level < kSahLevels ? 1 : 0, res);
-        k_plan_scan<<<1, 1024, 0, s>>>(cur, res, n, off, ctr);
-        k_plan_emit<<<grid_for(n, 128), 128, 0, s>>>(cur, res, n, off, nhid0, ncones0, nodes_used, q[(level & 1u) ^ 1u],
-                                                     plan.meta, plan.range, plan.up, plan.pair_at, plan.table);
-        g_launches += 3;
+        for (; ahead != 0u; --ahead) {
+            PlanNode* cur = q[level & 1u];
+            const PlanOut out = {nodes_used, q[(level & 1u) ^ 1u], plan.meta, plan.range, plan.up, np_at, plan.table};
+            // small ranges: one triangle or two a thread
+            const int threads = h.largest > 512u ? kPlanThreads : h.largest > 128u ? 128 : 64;
+            k_plan_split<<<most, threads, 0, s>>>(cur, plan.ids, tmp, cen, lo, hi, level < kSahLevels ? 1 : 0, res, ctr);
+            if (most <= 1024u) {
+                k_plan_scan<true><<<1, 1024, 0, s>>>(cur, res, off, out, ctr);
+                g_launches += 2;
+            } else {  // most is the level's own count: only small models queue ahead
+                k_plan_scan<false><<<1, 1024, 0, s>>>(cur, res, off, out, ctr);
+                k_plan_emit<<<grid_for(most, 128), 128, 0, s>>>(cur, res, most, off, h.nhid, h.ncones, out);
+                g_launches += 3;
+            }
+            most = std::min(4u * most, max_level);
+            ++level;
+        }
+        if (small) {
+            k_scan_tiles<<<tiles, 1024, 0, s>>>(np_at, ntris, plan.pair_at, plan.sums);
+            k_scan_sums<<<1, 1024, 0, s>>>(plan.sums, tiles, ctr);
+            g_launches += 2;
+        }
         if ((e = cudaMemcpyAsync(ctx->host_word, ctr, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
             (e = cudaStreamSynchronize(s)) != cudaSuccess)
             return e;
         h = *static_cast<const PlanCounters*>(ctx->host_word);
-        ++level;
+        most = h.nnext;
+        ahead = 1;
     }
-    k_scan_tiles<<<tiles, 1024, 0, s>>>(plan.pair_at, ntris, plan.sums);
-    k_scan_sums<<<1, 1024, 0, s>>>(plan.sums, tiles, ctr);
-    g_launches += 2;
-    if ((e = cudaMemcpyAsync(ctx->host_word, ctr, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-        return e;
-    h = *static_cast<const PlanCounters*>(ctx->host_word);
+    if (!small) {
+        k_scan_tiles<<<tiles, 1024, 0, s>>>(np_at, ntris, plan.pair_at, plan.sums);
+        k_scan_sums<<<1, 1024, 0, s>>>(plan.sums, tiles, ctr);
+        g_launches += 2;
+        if ((e = cudaMemcpyAsync(ctx->host_word, ctr, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(s)) != cudaSuccess)
+            return e;
+        h = *static_cast<const PlanCounters*>(ctx->host_word);
+    }
     plan.nhid = h.nhid;
     plan.nhp = h.nhp;
     plan.ncones = h.ncones;
-    plan.depth = level;
+    plan.depth = h.levels;
     return cudaGetLastError();
 }
 
 cudaError_t finish_hidden(bvhgpu_ctx* ctx, const HiddenPlan& plan, DeviceBlas& b, cudaStream_t s) {
     if (plan.nhid == 0u) return cudaSuccess;
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(b.hx, plan.table, 8ull * plan.table_u2, cudaMemcpyDeviceToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(b.hup, plan.up, 16ull * plan.nhid, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-        return e;
     LaunchScope scope(ctx, BVHGPU_K_OTHER, s);
-    k_plan_finish<<<grid_for(std::max(plan.nhid, b.nleaves), 128), 128, 0, s>>>(
-        plan.meta, plan.range, plan.nhid, plan.ids, plan.pair_at, plan.sums, pairs_in_order(b.ntris),
-        b.nodes + 2ull * b.nodes_used, b.hx + plan.table_u2, b.nodes, b.nodes_used, b.leaves, b.nleaves, plan.table,
-        b.hup + plan.nhid);
+    k_plan_finish<<<grid_for(std::max({plan.nhid, b.nleaves, plan.table_u2}), 128), 128, 0, s>>>(
+        plan.meta, plan.range, plan.up, plan.nhid, plan.ids, plan.pair_at, plan.sums, pairs_in_order(b.ntris),
+        b.nodes + 2ull * b.nodes_used, b.hup, b.hx + plan.table_u2, b.nodes, b.nodes_used, b.leaves, b.nleaves, plan.table,
+        plan.table_u2, b.hx);
     g_launches++;
     return cudaGetLastError();
 }

@@ -93,3 +93,21 @@ def test_leaves_of_a_built_bvh(ctx, n):
     check_plan(blas, [np.arange(l["left_first"], l["left_first"] + l["primitive_count"]) for l in leaves])
     trace(blas, bvh, tris, n, 12.0)
     blas.free()
+
+
+@pytest.mark.parametrize("kind", ["sphere", "spread"])
+def test_queued_levels_and_staging_memory(kind):
+    """Around the sizes up to which the levels are queued ahead and the work area is the context's staging
+    memory, in one fresh context and mixed with host traces that use and grow that memory; the models
+    uploaded first keep their hits."""
+    kept = []
+    with bt.Context(0) as ctx:
+        for n in (2048, 40, 2049, 4096, 16, 4097, 2047, 4095):
+            tris = shapes(kind, n)
+            bvh = one_leaf_bvh(tris)
+            blas = ctx.upload_blas(bvh, tris)
+            check_plan(blas, [np.arange(n)])
+            kept.append((blas, bvh, tris))
+            ctx.trace_batch(np.array([(blas.id, 0, 60000, 0)], bt.BATCH_ITEM), scenes.sphere_rays(60000, n, box=4.0), bt.MODE_PLAIN)
+        for blas, bvh, tris in kept:
+            trace(blas, bvh, tris, 5, 4.0)
