@@ -174,7 +174,8 @@ int bvhgpu_autotune(bvhgpu_ctx* ctx, const bvhgpu_tune_job* job, uint32_t reps, 
     };
     bvhgpu_tune_config cur = ctx->tune[j.kernel];
     if (!valid_config(cur)) cur = bvhgpu_tune_config{128u, 5u, 256u, 16u, 8u, 500u};
-    // start inside the search space: the margin limit moves to the nearest candidate
+    // search inside the space: the margin limit moves to the nearest candidate
+    const uint32_t given = cur.hidden;
     uint32_t hd = kHiddenValues[0];
     for (uint32_t h : kHiddenValues)
         if ((h > cur.hidden ? h - cur.hidden : cur.hidden - h) < (hd > cur.hidden ? hd - cur.hidden : cur.hidden - hd)) hd = h;
@@ -220,6 +221,22 @@ int bvhgpu_autotune(bvhgpu_ctx* ctx, const bvhgpu_tune_job* job, uint32_t reps, 
                 c.refill = rf;
                 consider(c);
             }
+        }
+    }
+    // a given limit outside the space comes back where it beats the winner by more than noise (the best of
+    // several runs in turn: models in large units can gain 1.7 times from 2000 over 1000)
+    if (given != hd && cur_ms < 3.0e38f) {
+        bvhgpu_tune_config own = cur;
+        own.hidden = given;
+        float a = 3.4e38f, b = 3.4e38f;
+        for (int r = 0; r < 5; ++r) {
+            const float x = measure(ctx, j, own, reps, tm), y = measure(ctx, j, cur, reps, tm);
+            if (x >= 0.0f) a = std::min(a, x);
+            if (y >= 0.0f) b = std::min(b, y);
+        }
+        if (a < 0.95f * b) {
+            cur = own;
+            cur_ms = a;
         }
     }
     ctx->tune[j.kernel] = cur;

@@ -502,7 +502,8 @@ typedef struct bvhgpu_tune_job {
     uint32_t nitems;
 } bvhgpu_tune_job;
 /* Times the job under candidate configs -- a coordinate search from the current config (its
- * hidden moved to the nearest candidate) over launch shape, stack, big_leaf, refill and hidden, two sweeps; each candidate runs once untimed, then
+ * hidden moved to the nearest candidate, and tried again at the end) over launch shape, stack,
+ * big_leaf, refill and hidden, two sweeps; each candidate runs once untimed, then
  * `reps` times bracketed by events on the context's stream (median kept) -- stores the fastest
  * in the context and returns it with its ms per call (either pointer may be NULL).  The job's
  * outputs are overwritten.  Synchronous; not allowed during graph capture. */
