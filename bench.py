@@ -236,20 +236,25 @@ def measured_peaks():
         return 6800.0, "fallback"
 
 
-def count_bytes(c: dict, n: int) -> int:
+# Bytes the traversal loads per hidden pair: its triangles, their indices in the pair's own last words.
+HIDDEN_PAIR_BYTES = 80
+
+
+def count_bytes(c: dict, n: int, pair: int = HIDDEN_PAIR_BYTES) -> int:
     """Node and triangle bytes the traversal fetched for n rays with work counters c (summed):
     64 B per reference interior node (its two children), 32 B per hidden child box, 40 B per
-    hidden-tree entry (table entry + root cone), 32 B per cone switch, 88 B per hidden pair (80 B
-    pair + 8 B slot indices), 48 / 40 B per triangle tested by a lane / the warp, 32 B ray + 20 B hit."""
+    hidden-tree entry (table entry + root cone), 32 B per cone switch, `pair` B per hidden pair,
+    48 / 40 B per triangle tested by a lane / the warp, 32 B ray + 20 B hit."""
     node_b = 64 * c["ref_nodes"] + 32 * c["hidden_boxes"] + 40 * c["hidden_entries"] + 32 * c["cone_switches"]
-    tri_b = 88 * c["hidden_pairs"] + 48 * c["lane_tris"] + 40 * c["warp_tris"]
+    tri_b = pair * c["hidden_pairs"] + 48 * c["lane_tris"] + 40 * c["warp_tris"]
     return node_b + tri_b + (32 + 20) * n
 
 
-def fetched_bytes(ctx, blas, rays, seed):
+def fetched_bytes(ctx, blas, rays, seed, pair=88):
     """Per-ray node and triangle bytes of the library's traversal, from bvhgpu_blas_trace_counts on
     the primaries and on their bounce rays (under the context's BVHGPU_K_TRACE_BLAS leaf policy:
-    call inside leaf_policy() to count another kernel's policy)."""
+    call inside leaf_policy() to count another kernel's policy).  pair: bytes per hidden pair (88 with
+    the slot indices in an array of their own, as the pairs were first laid out)."""
     import bvhtracer_gb300 as bt
     out = {}
     b_rays, valid = blas.bounce_rays(rays, seed)
@@ -258,7 +263,7 @@ def fetched_bytes(ctx, blas, rays, seed):
         d_r = ctx.to_device(rs)
         d_h = ctx.device_buffer(max(1, n) * bt.HIT.itemsize)
         c = blas.trace_counts(d_r, n, d_h)
-        total = count_bytes(c, n)
+        total = count_bytes(c, n, pair)
         out[key] = {"rays": n, "bytes": total, "bytes_per_ray": total / max(1, n),
                     "per_ray": {k: v / max(1, n) for k, v in c.items()}}
     return out
@@ -511,7 +516,7 @@ def bench_icosphere(args, pg=None):
     per_launch_s = dom_ms / dom_launches / 1e3
     policy_kernel = bt.K_PERSISTENT_BOUNCE if mode == bt.MODE_PERSISTENT else bt.K_TRACE_BLAS
     with leaf_policy(ctx, policy_kernel) as pol:
-        fetched = fetched_bytes(ctx, blas, rays, BOUNCE_SEED)
+        fetched = fetched_bytes(ctx, blas, rays, BOUNCE_SEED, HIDDEN_PAIR_BYTES)
     if mode == bt.MODE_PERSISTENT:
         own_bytes = fetched["primary"]["bytes"] + fetched["bounce"]["bytes"]
     else:
