@@ -79,15 +79,15 @@ struct GBlas {
     // Hidden trees of the large leaves (null when none): one uint2 per triangle index (rounded up
     // to even), read at a leaf's first triangle, {first, count} of the hidden root ({0, 0}: no
     // hidden tree); then one uint2 per hidden pair p >= (ntris + 1) / 2: the triangle indices of
-    // its two slots (0xFFFFFFFF: padding).  Hidden nodes follow the reference's nodes_used nodes in
+    // its two slots (0xFFFFFFFF: padding), which the refresh and the download read; the traversal
+    // has them in the pair's own last 8 bytes.  Hidden nodes follow the reference's nodes_used nodes in
     // `nodes` (a node whose children start at or beyond nodes_used is hidden): an interior one has
     // 2 to 4 children, consecutive from `first`, and count = kHiddenInterior | (children - 1) << 28 |
     // its cone; a leaf has count = kHiddenLeaf | pairs and first = its first pair in `pairs`, after
     // the (ntris + 1) / 2 pairs in triangle order.
     const uint2* hx;
     // Cone records of the hidden trees, 2 float4 each: {axis xyz, cos_phi}, {sin_phi, nmin, Q, B}
-    // (cull.cuh) -- one per hidden root and per hidden node at even depth; an interior hidden
-    // node's cone covers all its triangles.
+    // (cull.cuh) -- one per hidden root and per interior hidden node, covering all its triangles.
     const float4* cones;
     uint32_t nodes_used;
     uint32_t ntris;
@@ -101,10 +101,10 @@ constexpr uint32_t kConeMask = 0x0FFFFFFFu;
 constexpr uint32_t kWideShift = 28;  // hidden interior count: bits 28-29 = children - 1 (2..4 children)
 constexpr uint32_t kAnyCone = 0xFFFFFFFFu;  // TravT::lcone: the margins hold in the whole hidden tree
 // Below this root-cone margin a ray keeps the root cone's margins in the whole hidden tree (the
-// finer cones would cost more to evaluate than they save).  Measured at 0.5 | 0.05 (where it stood
-// with wider margins): soup frame 331 | 453 us, animated instanced frame 1,529 | 1,716, 512 x 512
-// Lambertian gradient 605 | 644, uneven batch 3,272 | 3,376; never switching: the same frames, but a
-// scene in large units (a sphere of radius 10 seen from 30) needs the finer cones.
+// finer cones would cost more to evaluate than they save).  Whole passes at 0.5 | 0.05, in us: full-HD frame with
+// bounces 892 | 890, soup frame 289 | 288, uneven batch 2,488 | 2,489, 512 x 512 Lambertian gradient 426 | 427,
+// animated instanced frame 1,546 | 1,548: any value there will do; a scene in large units (a sphere of radius
+// 10 seen from 30) needs the finer cones above it.
 constexpr float kConeSwitchDuv = 0.5f;
 
 // Whether a ray of barycentric margin duv walks the hidden tree of a leaf of n triangles whose normals span 60
@@ -124,13 +124,14 @@ __device__ __forceinline__ bool walk_soup(float duv, uint32_t n) { return duv * 
 __host__ __device__ __forceinline__ bool node_interior(uint32_t cnt) { return cnt == 0u || (cnt >> 30) == 1u; }
 __host__ __device__ __forceinline__ uint32_t hidden_table_u2(uint32_t ntris) { return (ntris + 1u) & ~1u; }
 // Reference leaves with at least this many triangles get a hidden tree, whose leaves hold at most
-// kHiddenLeafTris triangles (four packed pairs).  At 2 | 4 | 6 | 8 | 12 triangles, in us: full-HD frame with
-// bounces 764 | 790 | 765 | 786 | 823, soup frame 593 | 331 | 308 | 287 | 275, uneven batch 3,825 | 3,272 |
-// 2,848 | 2,785 | 2,638, Lambertian gradient 762 | 605 | 543 | 538 | 520, animated instanced frame 1,678 | 1,529 |
-// 1,538 | 1,548 | 1,583.
+// kHiddenLeafTris triangles (four packed pairs, one per lane of the refresh).  Whole passes at 4 | 6 | 8
+// triangles, in us: full-HD frame with bounces 896 | 862 | 892, soup frame 340 | 292 | 289, uneven batch 2,833 | 2,533 |
+// 2,488, 512 x 512 Lambertian gradient 441 | 416 | 426, animated instanced frame 1,512 | 1,509 | 1,546, scene image
+// 316 | 309 | 326.
 constexpr uint32_t kHiddenMinLeaf = 16;
 constexpr uint32_t kHiddenLeafTris = 8;
 static_assert(kHiddenMinLeaf > kHiddenLeafTris, "a hidden root is an interior node");
+static_assert(kHiddenLeafTris <= 8, "a quad of lanes refreshes a hidden leaf");
 
 __host__ __device__ __forceinline__ uint32_t pairs_in_order(uint32_t ntris) { return (ntris + 1u) / 2u; }
 

@@ -60,10 +60,8 @@
 // held an accepted hit at or below t_best, and the largest measured error was 0.21 of its margin (11.9 M hits).
 //
 // Counting the roundings term by term, instead of bounding each triple product by its largest
-// factors with a further factor 4 on every term, made R 50 to 100 times narrower.  With it hidden
-// trees pay for far rays and for soups too (measured, whole passes): uneven batch of 16 models
-// 11.0 -> 3.81 ms, animated instanced frame 11.2 -> 2.12 ms, 512 x 512 Lambertian gradient 1.56 ->
-// 0.77 ms, 24-instance image 633 -> 372 us, full-HD frame with bounces 1.05 -> 0.90 ms.
+// factors with a further factor 4 on every term, makes R 50 to 100 times and Du + Dv 3 to 9 times
+// narrower: hidden trees pay for far rays too.
 #pragma once
 
 #include <cfloat>
@@ -80,7 +78,8 @@ namespace bvhgpu {
 
 constexpr float kCullUnit = 5.9604645e-8f;  // u0 = 2^-24
 // A barycentric margin Du + Dv below which the bound from |det| >= 1e-4 is used as it is: the cone
-// would cost more to evaluate than its narrower margin saves (soup frame 453 us at 0.05, 399 at 0.5).
+// would cost more to evaluate than its narrower margin saves (at 0.5 | 0.05: animated instanced frame 1,546 | 1,562 us,
+// scene image 326 | 330, others the same).
 constexpr float kNarrowDuv = 0.5f;
 constexpr float kCullHuge = 1e15f;
 

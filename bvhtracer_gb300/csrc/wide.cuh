@@ -217,6 +217,9 @@ __device__ __forceinline__ bool wide_blas(const GBlas& g, LaneRay& r, LeafPolicy
 //               soup of 4,096             123 | 199 | 260 | 293 -> 24 | 39 | 81 | 134
 //  bounce, 320 / 5,120 / 81,920           67 | 59 | 64 | 66 -> 27 | 42 | 75 | 134;  120 | 119 | 122 | 120 ->
 //                                         35 | 56 | 100 | 181;  266 | 280 | 282 | 300 -> 49 | 75 | 134 | 237
+//  margins too wide to cull, all leaves in order: 20,000-triangle soup in units of 3 edges
+//                                         214 | 217 | 262 | 294 -> 44 | 69 | 122; sphere of 81,920, radius 100, 597 | 690 | 743 |
+//                                         952 -> 107 | 168 | 294 | 532
 //  Lambertian forward, 1,280 / 327,680    90 | 88 | 96 | 87 -> 19 | 30 | 53 | 96;  197 | 210 | 215 | 224 -> 30 | 46 | 82 | 144
 //  scene of 3 small objects               25 | 23 | 23 | 23 -> 15 | 19 | 27 | 44
 //  scene of 1,000 objects                 236 | 257 | 277 | 312 -> 47 | 72 | 126 | 226
