@@ -295,8 +295,8 @@ NCU_TRAFFIC = {
                           "profiles/k_persistent_bounce_icosphere_1080p_full.md"),
     "scene_bounce": (43.6e6 + 15.2e6, "ncu capture of one instanced 720p frame's trace launch",
                      "profiles/k_scene_persistent_bounce_instanced_720p_full.md"),
-    # 8-scene capture: 584.9 MB for 10,057,687 rays; scaled to a launch by its ray count
-    "trace_batch": (584.920064e6 / 10057687, "8-scene ncu capture, bytes per ray x rays",
+    # 8-scene capture: 650.2 MB for 10,057,687 rays; scaled to a launch by its ray count
+    "trace_batch": (650.156544e6 / 10057687, "8-scene ncu capture, bytes per ray x rays",
                     "profiles/k_trace_batch_persistent_64_scene_batch.md"),
 }
 
