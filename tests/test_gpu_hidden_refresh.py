@@ -7,6 +7,7 @@ import pytest
 
 import bvhtracer_gb300 as bt
 from bvhtracer_gb300 import scenes
+from oracle import oracle as orc
 from test_gpu_hidden import check_hidden_records, one_leaf_bvh
 
 pytestmark = pytest.mark.gpu
@@ -101,3 +102,46 @@ def test_root_cones_are_as_narrow_as_their_triangles(ctx, n, one):
             seen += 1
         assert seen >= (len(leaves) + 1) // 2 or (one and n > 100)
     blas.free()
+
+
+@pytest.mark.parametrize("level,scale", [(3, 100.0), (5, 100.0), (5, 1.0)])
+def test_mesh_update_measures_the_roots_in_its_refit(ctx, level, scale):
+    """A mesh update refreshes, then measures a large model's root cones in the refit's pass over the
+    triangles: the same cones as a vertex update of its own gives, and the oracle's refitted nodes, update after
+    update and replayed from a graph; a small model's roots stay valid cones."""
+    mesh = scenes.displaced_icosphere(level, 2)
+    verts = (mesh.vertices * np.float32(scale)).astype(np.float32)
+    m = bt.DiffMesh(ctx, verts, mesh.faces.astype(np.uint32), mesh.dirs.astype(np.float32))
+    nodes0, used = m.bvh.nodes.copy(), m.bvh.nodes_used
+    ctx.graph_begin()
+    m.update_async()
+    graph = ctx.graph_end()
+    for k in range(4):
+        verts = (verts * np.float32([1.0, 1.0 + 0.1 * k, 1.0])).astype(np.float32)
+        m.set_vertices(verts)
+        if k % 2:
+            m.update_async()
+        else:
+            ctx.graph_launch(graph)
+        ctx.sync()
+        tris = np.ascontiguousarray(verts[m.faces].reshape(-1, 9), np.float32)
+        check_hidden_records(m.blas, tris)
+        ref = orc.bvh_refit(nodes0, used, tris)[:used]
+        assert m.blas.download_nodes().tobytes() == ref.tobytes()
+        fused = m.blas.hidden_download()["cones"]
+        m.blas.update_vertices(tris)
+        assert m.blas.hidden_download()["cones"].tobytes() == fused.tobytes()
+        v = tris.reshape(-1, 3, 3)
+        e1, e2 = v[:, 1] - v[:, 0], v[:, 2] - v[:, 0]
+        table = m.blas.hidden_download()["table"]
+        leaves = [x for x in ref if x["primitive_count"] >= 16]
+        assert leaves
+        for leaf in leaves:
+            first, count = int(leaf["left_first"]), int(leaf["primitive_count"])
+            cone = fused[int(table[first, 1]) & 0x0FFFFFFF]
+            if cone[3] > 0:
+                least = least_cosine(e1[first:first + count], e2[first:first + count], cone[:3])
+                assert cone[3] == least if scale > 1 else cone[3] <= least
+    ctx.graph_free(graph)
+    ctx.lib.bvhgpu_mesh_free(ctx.h, m.id)
+    m.blas.free()
